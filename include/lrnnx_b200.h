@@ -79,7 +79,7 @@ typedef struct b200_selscan_fwd_args {
                                scanned from a zero state by its own thread blocks (more parallelism for
                                long rows); out, out_z and x of segments >= 1 are then zero-start results
                                that the caller must stitch with b200_selscan_fixup (n_segments = S).
-                               Honoured only on the shape class served by the throughput kernels,
+                               Honoured only on the shape class served by the state-parallel kernels,
                                rejected with B200_ERR_UNSUPPORTED elsewhere. */
   int32_t stage_len;        /* spacing in steps of the states in stage_h: the value returned by
                                b200_selscan_stage_states() for this problem (0 when stage_h is NULL) */
@@ -110,9 +110,9 @@ int b200_selscan_fwd(const b200_selscan_fwd_args *args, void *stream);
 
 /* Stage spacing (in steps) with which b200_selscan_fwd with these arguments (stage_h and
  * stage_len aside) would write stage_h and b200_selscan_bwd on the same problem would read it;
- * 0 if stage states are not used for this problem.  Non-zero on the shape class of the throughput
- * kernels with l_segments <= 1: 32 for the streaming kernels (enough rows to fill the GPU with
- * one warp per 16 channels), 256 for the lane-scan kernels. */
+ * 0 if stage states are not used for this problem.  Non-zero on the shape class of the
+ * state-parallel kernels with l_segments <= 1: 256, or 32 for problems of at least
+ * LRNNX_B200_SL_MIN_WARPS (environment variable) tiles of 16 channels. */
 int b200_selscan_stage_states(const b200_selscan_fwd_args *args);
 
 /* ------------------------------------------------------------------------
@@ -150,9 +150,18 @@ typedef struct b200_selscan_bwd_args {
    * of the loss with respect to the state after the last step, i.e. what later slices of the
    * sequence send back (b200_selscan_adjoint_summary, folded from the right). */
   const void *h_in, *q_in;
+  /* Device workspace of the state-parallel kernels, 32-byte aligned, free again when the call's work
+   * on `stream` is done: b200_selscan_bwd_work_bytes() bytes are enough (with fewer the batch is
+   * processed in thinner slices).  NULL: the call takes it from the stream-ordered allocator
+   * (cudaMallocAsync) and returns it on the same stream. */
+  void *work;
+  int64_t work_bytes;
 } b200_selscan_bwd_args;
 
 int b200_selscan_bwd(const b200_selscan_bwd_args *args, void *stream);
+
+/* Workspace of b200_selscan_bwd for these arguments; 0 where it uses none. */
+int64_t b200_selscan_bwd_work_bytes(const b200_selscan_bwd_args *args);
 
 /* ------------------------------------------------------------------------
  * Sequence-parallel helpers for the selective scan (no counterpart in lrnnx,

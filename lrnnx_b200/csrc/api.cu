@@ -42,7 +42,7 @@ using namespace b200;
 extern "C" {
 
 const char *b200_last_error(void) { return g_err; }
-int b200_abi_version(void) { return 5; }
+int b200_abi_version(void) { return 6; }
 
 // size of an argument block as this library was compiled; lets a binding
 // verify its own struct layout before the first call
@@ -72,18 +72,13 @@ int b200_selscan_fwd(const b200_selscan_fwd_args *args, void *stream) {
   B200_REQUIRE(args->out && args->x, B200_ERR_NULL, "selscan_fwd: out and x must be non-null");
   B200_REQUIRE(!args->z || args->out_z, B200_ERR_NULL, "selscan_fwd: out_z is required when z is given");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  // stage states are written only with the spacing the chosen kernel works in
-  b200_selscan_fwd_args a = *args;
-  if (selscan_fwd_sl_supported(a)) {
-    if (a.stage_len != kSlStage) a.stage_h = nullptr;
-    return selscan_fwd_sl(a, st);
-  }
-  if (selscan_fwd_fast_supported(a)) {
-    if (a.stage_len != kFastStage) a.stage_h = nullptr;
-    return selscan_fwd_fast(a, st);
+  if (selscan_seq_supported(*args)) {
+    b200_selscan_fwd_args a = *args;
+    if (a.stage_len <= 0 || a.stage_len % kStageUnit) a.stage_h = nullptr;     // stage states come in whole stages of the kernel
+    return selscan_seq_fwd(a, st);
   }
   B200_REQUIRE(args->l_segments <= 1, B200_ERR_UNSUPPORTED,
-               "selscan_fwd: l_segments > 1 is only available on the throughput-kernel shape class");
+               "selscan_fwd: l_segments > 1 is only available on the state-parallel kernels' shape class");
   return selscan_fwd_generic(*args, st);
 }
 
@@ -91,9 +86,12 @@ int b200_selscan_stage_states(const b200_selscan_fwd_args *args) {
   if (!args || check_selscan(*args) || args->l_segments > 1) return 0;
   b200_selscan_fwd_args a = *args;
   a.stage_h = nullptr;
-  if (selscan_fwd_sl_supported(a)) return kSlStage;
-  if (selscan_fwd_fast_supported(a)) return kFastStage;
-  return 0;
+  return selscan_seq_supported(a) ? selscan_seq_stage_len(a) : 0;
+}
+
+int64_t b200_selscan_bwd_work_bytes(const b200_selscan_bwd_args *args) {
+  if (!args || check_selscan(args->f) || !selscan_seq_bwd_supported(*args)) return 0;
+  return selscan_seq_bwd_bytes(args->f);
 }
 
 int b200_selscan_bwd(const b200_selscan_bwd_args *args, void *stream) {
@@ -111,17 +109,20 @@ int b200_selscan_bwd(const b200_selscan_bwd_args *args, void *stream) {
   B200_REQUIRE(!f.delta_bias || args->ddelta_bias, B200_ERR_NULL,
                "selscan_bwd: ddelta_bias is required when delta_bias is given");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (args->h_in || args->q_in) {      // a slice of a sequence-parallel backward: the coverage kernel takes both
-    B200_REQUIRE(!f.is_complex, B200_ERR_UNSUPPORTED, "selscan_bwd: h_in / q_in need a real A");
+  B200_REQUIRE(!(args->h_in || args->q_in) || !f.is_complex, B200_ERR_UNSUPPORTED, "selscan_bwd: h_in / q_in need a real A");
+  if (!selscan_seq_bwd_supported(*args)) return selscan_bwd_generic(*args, st);
+  b200_selscan_bwd_args a = *args;
+  if (a.f.stage_len <= 0 || kChunk % a.f.stage_len || a.f.stage_len % kStageUnit) a.f.stage_h = nullptr;
+  if (a.work) return selscan_seq_bwd(a, a.work, a.work_bytes, st);
+  void *work = nullptr;
+  const int64_t bytes = selscan_seq_bwd_bytes(f);
+  if (cudaMallocAsync(&work, (size_t)bytes, st) != cudaSuccess) {
+    cudaGetLastError();                       // no room for the workspace: the coverage kernel needs none
     return selscan_bwd_generic(*args, st);
   }
-  if (selscan_bwd_sl_supported(*args)) return selscan_bwd_sl(*args, st);
-  if (selscan_bwd_fast_supported(*args)) {
-    b200_selscan_bwd_args a = *args;
-    if (a.f.stage_len != kFastStage) a.f.stage_h = nullptr;    // states of another spacing: recompute
-    return selscan_bwd_fast(a, st);
-  }
-  return selscan_bwd_generic(*args, st);
+  const int e = selscan_seq_bwd(a, work, bytes, st);
+  cudaFreeAsync(work, st);
+  return e;
 }
 
 }  // extern "C"

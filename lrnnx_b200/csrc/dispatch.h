@@ -5,24 +5,19 @@
 
 namespace b200 {
 
-constexpr int kSlStage = 32;      // stage_h spacing of the streaming kernels (selscan_sl.cu)
-constexpr int kFastStage = 256;   // stage_h spacing of the lane-scan kernels (selscan_fast.cu)
+constexpr int kStageUnit = 32;    // stage_h spacings of the state-parallel kernels are multiples of this
 
 // coverage kernels: every variant (selscan_generic.cu)
 int selscan_fwd_generic(const b200_selscan_fwd_args &a, cudaStream_t st);
 int selscan_bwd_generic(const b200_selscan_bwd_args &a, cudaStream_t st);
 
-// throughput kernels for the hot S6 shape class (selscan_fast.cu)
-bool selscan_fwd_fast_supported(const b200_selscan_fwd_args &a);
-bool selscan_bwd_fast_supported(const b200_selscan_bwd_args &a);
-int selscan_fwd_fast(const b200_selscan_fwd_args &a, cudaStream_t st);
-int selscan_bwd_fast(const b200_selscan_bwd_args &a, cudaStream_t st);
-
-// streaming kernels for the same shape class when there are enough rows (selscan_sl.cu)
-bool selscan_fwd_sl_supported(const b200_selscan_fwd_args &a);
-bool selscan_bwd_sl_supported(const b200_selscan_bwd_args &a);
-int selscan_fwd_sl(const b200_selscan_fwd_args &a, cudaStream_t st);
-int selscan_bwd_sl(const b200_selscan_bwd_args &a, cudaStream_t st);
+// state-parallel kernels (selscan_seq.cu, selscan_seq_bwd.cu)
+bool selscan_seq_supported(const b200_selscan_fwd_args &a);
+int selscan_seq_stage_len(const b200_selscan_fwd_args &a);
+int selscan_seq_fwd(const b200_selscan_fwd_args &a, cudaStream_t st);
+bool selscan_seq_bwd_supported(const b200_selscan_bwd_args &a);
+int64_t selscan_seq_bwd_bytes(const b200_selscan_fwd_args &f);
+int selscan_seq_bwd(const b200_selscan_bwd_args &a, void *work, int64_t work_bytes, cudaStream_t st);
 
 // status word of the tensor-core projection kernel (cgemm_tc.cu)
 int cgemm_status_read();

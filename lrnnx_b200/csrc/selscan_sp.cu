@@ -143,8 +143,7 @@ __global__ void __launch_bounds__(SPW * 32) selscan_fixup_kernel(const b200_sels
 
 // ---- vectorized variant: 8 consecutive timesteps per lane (256 per iteration), 16-byte typed
 // loads and stores.  Needs 16-byte aligned rows, a sequence length and segment starts that are
-// multiples of 8 — what the throughput forward kernel, the only producer of in-GPU segments,
-// requires as well.
+// multiples of 8.
 template <typename T> struct V8;
 template <> struct V8<float> {
   __device__ static void load(const float *p, float (&v)[8]) {

@@ -131,37 +131,38 @@ _SM_COUNT = {}
 
 def _segments_for(u, batch, dim, seqlen, dstate, n_groups, is_complex, var_B, var_C, deltaA, method):
     """Number of sequence segments for the forward call: > 1 only for long rows that would leave
-    most of the GPU idle (few (batch, channel-tile) thread blocks), on the shape class of the
-    throughput kernel.  Segments are scanned concurrently from zero states and stitched by the
-    summary fold + fix-up that the multi-GPU sequence-parallel path uses."""
+    part of the GPU idle, on the shape class of the state-parallel kernels.  Segments are scanned
+    concurrently from zero states and stitched by the summary fold + fix-up that the multi-GPU
+    sequence-parallel path uses."""
     if is_complex or method != "mamba" or not (var_B and var_C) or deltaA is not None or dstate != 16:
         return 1
-    if dim % 16 or (dim // n_groups) % 16 or seqlen % 8 or seqlen < 4 * CHUNK:
+    if seqlen < 4 * CHUNK:
         return 1
     idx = u.device.index if u.device.index is not None else torch.cuda.current_device()
     if idx not in _SM_COUNT:
         _SM_COUNT[idx] = torch.cuda.get_device_properties(idx).multi_processor_count
-    slots = 8 * _SM_COUNT[idx]     # resident 16-channel warp tiles of the streaming kernel
-    ctas = batch * dim // 16
-    if ctas >= 4 * slots:
+    sms = _SM_COUNT[idx]
+    rows = batch * dim
+    ctas = batch * n_groups * -(-(dim // n_groups) // 32)       # thread blocks of 32 channels; 3 fit on an SM
+    if ctas >= 12 * sms:
         return 1
-    # pick the segment count whose thread blocks fill whole waves best (ties: fewer segments)
-    best, best_eff = 1, 0.0
+    # measured: a step of a thread block takes 60, 80 and 105 ns with one, two and three of them on an SM;
+    # the fix-up of a segment takes 6 ns per row
+    step_ns = (0, 60, 80, 105)
+    best, best_ns = 1, None
     for want in range(1, 17):
         seg_len = -(-(-(-seqlen // want)) // CHUNK) * CHUNK
         if want > 1 and seg_len < 2 * CHUNK:
             break
         S = -(-seqlen // seg_len)
-        waves = ctas * S / slots
-        # below one wave more segments simply mean more of the GPU in use; above, whole waves count.
-        # Every extra segment also costs a fix-up pass over its first steps: demand a clear gain.
-        eff = waves if waves <= 1.0 else waves / -(-waves // 1)
-        if eff > best_eff * 1.10 + 1e-9:
-            best, best_eff = S, eff
+        full, rest = divmod(ctas * S, 3 * sms)
+        ns = (full * step_ns[3] + step_ns[-(-rest // sms)]) * seg_len + 6 * rows * (S - 1)
+        if best_ns is None or ns < 0.95 * best_ns:
+            best, best_ns = S, ns
     return best
 
 
-# Stage states: the throughput kernels pass the state at every stage boundary from the forward to
+# Stage states: the state-parallel kernels pass the state at every stage boundary from the forward to
 # the backward call (which then skips recomputing them).  They live behind the checkpoints in x's
 # own allocation, so the reference's fwd / bwd signatures stay as they are.  bwd() recognises an x
 # made by fwd() through a registry of weak references to the storages fwd() allocated (a copy, a
@@ -245,7 +246,7 @@ def fwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, delta_softplus, discret
             except RuntimeError as e:
                 if "l_segments" not in str(e):
                     raise
-                S, a.l_segments = 1, 0       # operands not aligned for the throughput kernel
+                S, a.l_segments = 1, 0       # operands that the state-parallel kernels do not take
                 _lib.call("b200_selscan_fwd", a, _stream(u))
             if S > 1:
                 _stitch_segments(a, x, S, seqlen, u)
@@ -345,6 +346,10 @@ def bwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, dout, x_, out_, dz_, de
             q.dC_bs, q.dC_gs, q.dC_ns = dC.stride(0), dC.stride(1), dC.stride(2)
         else:
             q.dC_bs, q.dC_gs, q.dC_ns = 0, dC.stride(0), dC.stride(1)
+        work_bytes = _lib.lib().b200_selscan_bwd_work_bytes(ctypes.byref(q))
+        if work_bytes > 0:
+            work = torch.empty(work_bytes, dtype=torch.uint8, device=u.device)
+            q.work, q.work_bytes = work.data_ptr(), work_bytes
         _lib.call("b200_selscan_bwd", q, _stream(u))
         result = [du, ddelta, dA, dB.to(B.dtype), dC.to(C.dtype), dD, ddelta_bias]
         if deltaA_ is not None:

@@ -1,0 +1,91 @@
+"""The state-parallel selective-scan kernels where their tilings can go wrong: channel counts that leave a
+warp (8 channels), a thread block (32) or a group partly empty, lengths around the 4-step blocks, the
+32-step stages, the 128-step windows, the 256-step pieces and the 2048-step checkpoints, rows that are not
+16-byte aligned, and the three ways the backward gets its states and its workspace."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from conftest import assert_close
+from oracle import scan_oracle as O
+from test_gpu_selective_scan import ATOL32, GRAD_ATOL32, GRAD_RTOL32, RTOL32, _make_inputs
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1, 8, 1, 1), (2, 3, 3, 1), (1, 33, 31, 1), (2, 40, 32, 2), (1, 24, 33, 3), (2, 72, 127, 1), (1, 16, 129, 2),
+          (1, 5, 257, 1), (2, 34, 513, 2), (1, 8, 2047, 1), (1, 9, 2049, 1), (1, 12, 4100, 2)]
+
+
+def _grads(t, kw, gout, fn):
+    leaves = {k: (v.detach().clone().requires_grad_(True) if torch.is_tensor(v) else v) for k, v in t.items()}
+    out = fn(**leaves, **kw)
+    names = [k for k, v in leaves.items() if torch.is_tensor(v)]
+    return out.detach(), dict(zip(names, torch.autograd.grad(out, [leaves[k] for k in names], gout)))
+
+
+@pytest.mark.parametrize("batch,dim,L,groups", SHAPES)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_edges_of_the_tilings(batch, dim, L, groups, dtype):
+    from lrnnx_b200.ops import selective_scan_fn
+    t, g = _make_inputs(batch, dim, 16, L, seed=L + dim, dtype=dtype, groups=groups, with_z=L % 2 == 1)
+    kw = dict(delta_softplus=True, discretization="mamba")
+    gout = torch.randn(batch, dim, L, generator=g).to(dtype)
+    out_c, gc = _grads(t, kw, gout, O.selective_scan_oracle)
+    out_g, gg = _grads({k: (v.cuda() if torch.is_tensor(v) else v) for k, v in t.items()}, kw, gout.cuda(), selective_scan_fn)
+    f32 = dtype == torch.float32
+    assert_close(out_g.float().cpu(), out_c.float(), rtol=RTOL32 if f32 else 3e-2, atol_scale=ATOL32 if f32 else 1e-2, name="out")
+    for k in gc:
+        assert_close(gg[k].float().cpu(), gc[k].float(), rtol=GRAD_RTOL32 if f32 else 3e-2, atol_scale=GRAD_ATOL32 if f32 else 2e-2, name=f"d{k}")
+
+
+@pytest.mark.parametrize("offset", [1, 2, 4])
+def test_rows_that_are_not_16_byte_aligned(offset):
+    """The same operands as dense tensors and as views that start `offset` elements into wider rows take different
+    load paths of the same kernels: outputs are equal bit for bit, gradients up to the order of the atomics."""
+    from lrnnx_b200.ops import selective_scan_fn
+    t, g = _make_inputs(2, 40, 16, 264, seed=5)
+    dense = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in t.items()}
+    views = dict(dense)
+    for k in ("u", "delta", "z", "B", "C"):
+        wide = torch.full((*dense[k].shape[:-1], 264 + 9), float("nan"), device="cuda")
+        wide[..., offset:offset + 264] = dense[k]
+        views[k] = wide[..., offset:offset + 264]
+    kw = dict(delta_softplus=True, discretization="mamba")
+    gout = torch.randn(2, 40, 264, generator=g).cuda()
+
+    def run(ops):
+        leaves = {k: (v.detach().requires_grad_(True) if torch.is_tensor(v) else v) for k, v in ops.items()}
+        out = selective_scan_fn(**leaves, **kw)
+        return out.detach(), torch.autograd.grad(out, [v for v in leaves.values() if torch.is_tensor(v)], gout)
+
+    (out_a, ga), (out_b, gb) = run(dense), run(views)
+    assert torch.equal(out_a, out_b)
+    for a, b in zip(ga, gb):
+        assert_close(b.cpu(), a.cpu(), rtol=1e-5, atol_scale=1e-6, name="gradient")
+
+
+@pytest.mark.parametrize("L", [200, 4200])
+def test_backward_workspaces(L, monkeypatch):
+    """The workspace for the whole batch, for one batch row at a time, and none (the call takes its own): the same
+    gradients; and the states rebuilt from the checkpoints alone (an x that did not come from fwd) agree as well."""
+    from lrnnx_b200 import _lib
+    from lrnnx_b200 import selective_scan_cuda as ext
+    t, g = _make_inputs(3, 24, 16, L, seed=L)
+    c = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in t.items()}
+    args = (c["u"], c["delta"], c["A"], c["B"], c["C"], c["D"], c["z"], c["delta_bias"], None)
+    out, x, _ = ext.fwd(*args, True, "mamba")
+    dout = torch.randn(out.shape, generator=g).cuda()
+    want = ext.bwd(*args, dout, x, out, None, True, False, "mamba")
+    call = _lib.call
+    for mode in ("row", "none", "checkpoints"):
+        def patched(fn, a, stream, mode=mode):
+            if fn == "b200_selscan_bwd" and mode == "row":
+                a.work_bytes //= 3
+            if fn == "b200_selscan_bwd" and mode == "none":
+                a.work = None
+            call(fn, a, stream)
+        monkeypatch.setattr(_lib, "call", patched)
+        got = ext.bwd(*args, dout, x.clone() if mode == "checkpoints" else x, out, None, True, False, "mamba")
+        for i, (a, b) in enumerate(zip(got, want)):
+            assert_close(a.cpu(), b.cpu(), rtol=2e-5, atol_scale=2e-6, name=f"{mode} gradient {i}")

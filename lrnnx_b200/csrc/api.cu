@@ -79,6 +79,7 @@ int b200_selscan_fwd(const b200_selscan_fwd_args *args, void *stream) {
   }
   B200_REQUIRE(args->l_segments <= 1, B200_ERR_UNSUPPORTED,
                "selscan_fwd: l_segments > 1 is only available on the state-parallel kernels' shape class");
+  if (selscan_row1_supported(*args)) return selscan_row1_fwd(*args, st);
   return selscan_fwd_generic(*args, st);
 }
 
@@ -110,6 +111,7 @@ int b200_selscan_bwd(const b200_selscan_bwd_args *args, void *stream) {
                "selscan_bwd: ddelta_bias is required when delta_bias is given");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   B200_REQUIRE(!(args->h_in || args->q_in) || !f.is_complex, B200_ERR_UNSUPPORTED, "selscan_bwd: h_in / q_in need a real A");
+  if (!args->h_in && !args->q_in && selscan_row1_supported(f)) return selscan_row1_bwd(*args, st);
   if (!selscan_seq_bwd_supported(*args)) return selscan_bwd_generic(*args, st);
   b200_selscan_bwd_args a = *args;
   if (a.f.stage_len <= 0 || kChunk % a.f.stage_len || a.f.stage_len % kStageUnit) a.f.stage_h = nullptr;

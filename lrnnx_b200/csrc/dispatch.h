@@ -19,6 +19,11 @@ bool selscan_seq_bwd_supported(const b200_selscan_bwd_args &a);
 int64_t selscan_seq_bwd_bytes(const b200_selscan_fwd_args &f);
 int selscan_seq_bwd(const b200_selscan_bwd_args &a, void *work, int64_t work_bytes, cudaStream_t st);
 
+// one state per channel, constant B and C: RG-LRU and S7 (selscan_row1.cu)
+bool selscan_row1_supported(const b200_selscan_fwd_args &a);
+int selscan_row1_fwd(const b200_selscan_fwd_args &a, cudaStream_t st);
+int selscan_row1_bwd(const b200_selscan_bwd_args &a, cudaStream_t st);
+
 // status word of the tensor-core projection kernel (cgemm_tc.cu)
 int cgemm_status_read();
 

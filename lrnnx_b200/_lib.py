@@ -14,6 +14,8 @@ import re
 from functools import lru_cache
 from pathlib import Path
 
+import torch
+
 _PKG = Path(__file__).resolve().parent
 HEADER = _PKG.parent / "include" / "lrnnx_b200.h"
 LIB_PATH = _PKG / "lib" / "liblrnnx_b200.so"
@@ -135,6 +137,27 @@ def check_layout() -> None:
         want = _lib.b200_sizeof(name.encode())
         if want != ctypes.sizeof(st):
             raise RuntimeError(f"ABI mismatch for {name}: header says {ctypes.sizeof(st)} bytes, library {want}")
+
+
+class _SameDevice:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_SAME_DEVICE = _SameDevice()
+
+
+def on_device(t):
+    """``torch.cuda.device(t.device)``, without the switch where that device is current already."""
+    return _SAME_DEVICE if t.device.index == torch.cuda.current_device() else torch.cuda.device(t.device)
+
+
+def stream_of(t) -> int:
+    """The raw handle of the current stream on t's device."""
+    return torch._C._cuda_getCurrentRawStream(t.device.index)
 
 
 def call(fn_name: str, args: ctypes.Structure, stream: int) -> None:

@@ -29,7 +29,7 @@ class CrossEntropyFn(torch.autograd.Function):
         a.rows, a.cols = logits.shape
         a.dtype = _lib.enum(_DT[logits.dtype])
         a.ignore_index = ignore_index
-        with torch.cuda.device(logits.device):
+        with _lib.on_device(logits):
             lse = torch.empty(logits.shape[0], dtype=torch.float32, device=logits.device)
             loss = torch.empty_like(lse)
             a.logits, a.labels, a.lse, a.loss = logits.data_ptr(), labels.data_ptr(), lse.data_ptr(), loss.data_ptr()
@@ -48,7 +48,7 @@ class CrossEntropyFn(torch.autograd.Function):
         a.rows, a.cols = logits.shape
         a.dtype = _lib.enum(_DT[logits.dtype])
         a.ignore_index = ctx.ignore_index
-        with torch.cuda.device(logits.device):
+        with _lib.on_device(logits):
             scale = (grad.to(torch.float32) / counted).reshape(1).contiguous()
             dlogits = torch.empty_like(logits)
             a.logits, a.labels, a.lse = logits.data_ptr(), labels.data_ptr(), lse.data_ptr()

@@ -43,7 +43,7 @@ def linear_step(x, weight, bias=None):
     a.M, a.K = x.shape
     a.N = weight.shape[0]
     a.dtype = _lib.enum(_DT[x.dtype])
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x):
         out = torch.empty(x.shape[0], weight.shape[0], dtype=x.dtype, device=x.device)
         a.x, a.weight, a.out = x.data_ptr(), weight.data_ptr(), out.data_ptr()
         a.bias = None if bias is None else bias.contiguous().data_ptr()

@@ -18,7 +18,7 @@ _DT = {torch.float32: "B200_F32", torch.float16: "B200_F16", torch.bfloat16: "B2
 
 
 def _stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _lib.stream_of(t)
 
 
 def _conv_args(x, weight, bias, silu):
@@ -46,7 +46,7 @@ class CausalConv1dFn(torch.autograd.Function):
         b = None if bias is None else bias.to(x.dtype).contiguous()
         a = _conv_args(x, w, b, silu)
         a.batch, _, a.seqlen = x.shape
-        with torch.cuda.device(x.device):
+        with _lib.on_device(x):
             out = torch.empty_like(x, memory_format=torch.contiguous_format)
             a.x, a.out = x.data_ptr(), out.data_ptr()
             a.x_bs, a.x_ds = x.stride(0), x.stride(1)
@@ -65,7 +65,7 @@ class CausalConv1dFn(torch.autograd.Function):
             dout = dout.contiguous()
         a = _conv_args(x, w, b, ctx.silu)
         a.batch, _, a.seqlen = x.shape
-        with torch.cuda.device(x.device):
+        with _lib.on_device(x):
             dx = torch.empty_like(x, memory_format=torch.contiguous_format)
             dw = torch.zeros(w.shape, dtype=torch.float32, device=x.device)
             db = torch.zeros(w.shape[0], dtype=torch.float32, device=x.device) if b is not None else None
@@ -98,7 +98,7 @@ def causal_conv1d_update(x, conv_state, weight, bias=None, activation=None):
     a = _conv_args(x, w, b, activation is not None)
     a.batch = x.shape[0]
     a.seqlen = 1
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x):
         out = torch.empty_like(x)
         a.x, a.out, a.state = x.data_ptr(), out.data_ptr(), conv_state.data_ptr()
         a.x_bs, a.x_ds = x.stride(0), x.stride(1)
@@ -129,7 +129,7 @@ class RMSNormFn(torch.autograd.Function):
         a.rows, a.cols = x2.shape
         a.dtype, a.residual_dtype = _lib.enum(_DT[x.dtype]), _lib.enum(_DT[rdtype])
         a.eps = eps
-        with torch.cuda.device(x.device):
+        with _lib.on_device(x):
             y = torch.empty_like(x2)
             z = torch.empty(x2.shape, dtype=rdtype, device=x.device)     # x + residual: output of prenorm, input of backward
             rstd = torch.empty(x2.shape[0], dtype=torch.float32, device=x.device)
@@ -162,7 +162,7 @@ class RMSNormFn(torch.autograd.Function):
         a.rows, a.cols = z.shape
         a.dtype, a.residual_dtype = _lib.enum(_DT[xdtype]), _lib.enum(_DT[rdtype])
         a.eps = eps
-        with torch.cuda.device(z.device):
+        with _lib.on_device(z):
             dx = torch.empty(z.shape, dtype=xdtype, device=z.device)
             dres_in = torch.empty(z.shape, dtype=rdtype, device=z.device) if (has_residual and rdtype != xdtype) else None
             dw = torch.zeros(z.shape[1], dtype=torch.float32, device=z.device)

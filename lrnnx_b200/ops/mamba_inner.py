@@ -57,7 +57,7 @@ class MambaInnerFn(torch.autograd.Function):
         dt = xz.dtype
         w2 = conv1d_weight.reshape(d, -1).to(dt).contiguous()
         cb = None if conv1d_bias is None else conv1d_bias.to(dt).contiguous()
-        with torch.cuda.device(xz.device):
+        with _lib.on_device(xz):
             x, z = xz[:, :d], xz[:, d:]
             xc = _conv_forward(x, w2, cb)
             x_dbl = torch.bmm(_wb(x_proj_weight.to(dt), batch), xc)                    # (batch, R + 2N, L)
@@ -84,7 +84,7 @@ class MambaInnerFn(torch.autograd.Function):
         N = A.shape[1]
         R = delta_proj_weight.shape[1]
         dt = xz.dtype
-        with torch.cuda.device(xz.device):
+        with _lib.on_device(xz):
             x, z = xz[:, :d], xz[:, d:]
             dy = dy.to(dt)
             # out_proj

@@ -34,10 +34,10 @@ def weight_planes(W, conj_transpose=False):
     a = _lib.struct("b200_cgemm_planes_args")()
     a.M, a.K, a.conj = M, K, int(conj_transpose)
     a.w_rs, a.w_cs = (W.stride(1), W.stride(0)) if conj_transpose else (W.stride(0), W.stride(1))
-    with torch.cuda.device(W.device):
+    with _lib.on_device(W):
         planes = torch.empty((4, M, K), dtype=torch.float32, device=W.device)
         a.w, a.planes = W.data_ptr(), planes.data_ptr()
-        _lib.call("b200_cgemm_planes", a, torch.cuda.current_stream(W.device).cuda_stream)
+        _lib.call("b200_cgemm_planes", a, _lib.stream_of(W))
     return planes
 
 
@@ -52,12 +52,12 @@ def project(W, x, conj_transpose=False):
         x = x.contiguous()
     a = _lib.struct("b200_cgemm_args")()
     a.batch, a.M, a.K, a.N = batch, M, K, N
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x):
         out = torch.empty((batch, M, N), dtype=torch.complex64, device=x.device)
         a.w_planes, a.x, a.out = planes.data_ptr(), x.data_ptr(), out.data_ptr()
         a.x_bs, a.x_ks = x.stride(0), x.stride(1)
         a.out_bs, a.out_ms = out.stride(0), out.stride(1)
-        _lib.call("b200_cgemm_wx", a, torch.cuda.current_stream(x.device).cuda_stream)
+        _lib.call("b200_cgemm_wx", a, _lib.stream_of(x))
     return out
 
 
@@ -79,8 +79,8 @@ def weight_grad(g, u):
     a = _lib.struct("b200_cgemm_grad_args")()
     a.batch, a.M, a.L = g.shape
     a.N = u.shape[1]
-    with torch.cuda.device(g.device):
+    with _lib.on_device(g):
         out = torch.zeros((g.shape[1], u.shape[1]), dtype=torch.complex64, device=g.device)
         a.g, a.u, a.out = g.data_ptr(), u.data_ptr(), out.data_ptr()
-        _lib.call("b200_cgemm_grad", a, torch.cuda.current_stream(g.device).cuda_stream)
+        _lib.call("b200_cgemm_grad", a, _lib.stream_of(g))
     return out

@@ -51,7 +51,7 @@ def simplified_state_update(state, x, dt, A, B, C, D=None, deltaA=None, discreti
     a.conj_sym = int(bool(conj_sym))
     A, B, C = A.contiguous(), B.contiguous(), C.contiguous()
     keep = [dt, A, B, C, x]
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x):
         out = torch.empty((batch, H), dtype=torch.float32, device=x.device)
         a.state, a.x, a.dt, a.A, a.B, a.C, a.out = (state.data_ptr(), x.data_ptr(), dt.data_ptr(), A.data_ptr(),
                                                     B.data_ptr(), C.data_ptr(), out.data_ptr())
@@ -64,5 +64,5 @@ def simplified_state_update(state, x, dt, A, B, C, D=None, deltaA=None, discreti
             D = D.float().contiguous()
             keep.append(D)
             a.D = D.data_ptr()
-        _lib.call("b200_s5_step", a, torch.cuda.current_stream(x.device).cuda_stream)
+        _lib.call("b200_s5_step", a, _lib.stream_of(x))
     return out

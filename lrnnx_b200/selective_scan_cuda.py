@@ -12,8 +12,10 @@ recurrence state is always fp32.
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
+from torch.multiprocessing.reductions import StorageWeakRef
 
 from . import _lib
 
@@ -34,12 +36,16 @@ def _check(cond: bool, msg: str) -> None:
         raise RuntimeError(msg)
 
 
+_code = functools.lru_cache(maxsize=None)(_lib.enum)
+
+
 def _ptr(t):
     return None if t is None else t.data_ptr()
 
 
 def _shape(t, *shape, name: str) -> None:
-    _check(tuple(t.shape) == tuple(shape), f"{name} must have shape {tuple(shape)}, got {tuple(t.shape)}")
+    if t.shape != shape:
+        raise RuntimeError(f"{name} must have shape {tuple(shape)}, got {tuple(t.shape)}")
 
 
 def _common(u, delta, A, B, C, D, z, delta_bias, deltaA, discretization):
@@ -57,7 +63,8 @@ def _common(u, delta, A, B, C, D, z, delta_bias, deltaA, discretization):
     _check(B.dtype == (u.dtype if var_B else A.dtype), "B has the wrong dtype")
     _check(C.dtype == (u.dtype if var_C else A.dtype), "C has the wrong dtype")
     for name, t in (("u", u), ("delta", delta), ("A", A), ("B", B), ("C", C)):
-        _check(t.is_cuda, f"{name} must be a CUDA tensor")
+        if not t.is_cuda:
+            raise RuntimeError(f"{name} must be a CUDA tensor")
     _check(u.dim() == 3, "u must be (batch, dim, seqlen)")
     _check(u.stride(-1) == 1 or u.size(-1) == 1, "u must be contiguous in the last dimension")
     _check(delta.stride(-1) == 1 or delta.size(-1) == 1, "delta must be contiguous in the last dimension")
@@ -85,47 +92,46 @@ def _common(u, delta, A, B, C, D, z, delta_bias, deltaA, discretization):
     _check(dim % n_groups == 0, "dim must be a multiple of the number of groups")
     for name, t in (("D", D), ("delta_bias", delta_bias)):
         if t is not None:
-            _check(t.dtype == torch.float32, f"{name} must be float32")
-            _check(t.is_cuda, f"{name} must be a CUDA tensor")
-            _check(t.stride(-1) == 1 or t.size(-1) == 1, f"{name} must be contiguous")
+            if t.dtype != torch.float32 or not t.is_cuda or not (t.stride(-1) == 1 or t.size(-1) == 1):
+                _check(t.dtype == torch.float32, f"{name} must be float32")
+                _check(t.is_cuda, f"{name} must be a CUDA tensor")
+                raise RuntimeError(f"{name} must be contiguous")
             _shape(t, dim, name=name)
     for name, t in (("deltaA", deltaA), ("z", z)):
         if t is not None:
-            _check(t.dtype == u.dtype, f"{name} must have the dtype of u")
-            _check(t.is_cuda, f"{name} must be a CUDA tensor")
-            _check(t.stride(-1) == 1 or t.size(-1) == 1, f"{name} must be contiguous in the last dimension")
+            if t.dtype != u.dtype or not t.is_cuda or not (t.stride(-1) == 1 or t.size(-1) == 1):
+                _check(t.dtype == u.dtype, f"{name} must have the dtype of u")
+                _check(t.is_cuda, f"{name} must be a CUDA tensor")
+                raise RuntimeError(f"{name} must be contiguous in the last dimension")
             _shape(t, batch, dim, seqlen, name=name)
 
     a = _lib.struct("b200_selscan_fwd_args")()
     a.batch, a.dim, a.seqlen, a.dstate, a.n_groups = batch, dim, seqlen, dstate, n_groups
-    a.dtype = _lib.enum(_DTYPES[u.dtype])
+    a.dtype = _code(_DTYPES[u.dtype])
     a.is_complex = int(is_complex)
     a.var_B, a.var_C = int(var_B), int(var_C)
-    a.method = _lib.enum(_METHODS[discretization])
+    a.method = _code(_METHODS[discretization])
     a.u, a.delta, a.A, a.B, a.C = u.data_ptr(), delta.data_ptr(), A.data_ptr(), B.data_ptr(), C.data_ptr()
     a.D, a.z, a.delta_bias, a.deltaA = _ptr(D), _ptr(z), _ptr(delta_bias), _ptr(deltaA)
-    a.u_bs, a.u_ds = u.stride(0), u.stride(1)
-    a.delta_bs, a.delta_ds = delta.stride(0), delta.stride(1)
+    a.u_bs, a.u_ds, _ = u.stride()
+    a.delta_bs, a.delta_ds, _ = delta.stride()
     if z is not None:
-        a.z_bs, a.z_ds = z.stride(0), z.stride(1)
+        a.z_bs, a.z_ds, _ = z.stride()
     if deltaA is not None:
-        a.deltaA_bs, a.deltaA_ds = deltaA.stride(0), deltaA.stride(1)
-    a.A_ds, a.A_ns = A.stride(0), A.stride(1)
+        a.deltaA_bs, a.deltaA_ds, _ = deltaA.stride()
+    a.A_ds, a.A_ns = A.stride()
     if var_B:
-        a.B_bs, a.B_gs, a.B_ns = B.stride(0), B.stride(1), B.stride(2)
+        a.B_bs, a.B_gs, a.B_ns, _ = B.stride()
     else:
-        a.B_bs, a.B_gs, a.B_ns = 0, B.stride(0), B.stride(1)
+        a.B_gs, a.B_ns = B.stride()
     if var_C:
-        a.C_bs, a.C_gs, a.C_ns = C.stride(0), C.stride(1), C.stride(2)
+        a.C_bs, a.C_gs, a.C_ns, _ = C.stride()
     else:
-        a.C_bs, a.C_gs, a.C_ns = 0, C.stride(0), C.stride(1)
+        a.C_gs, a.C_ns = C.stride()
     return a, (batch, dim, seqlen, dstate, n_groups, is_complex, var_B, var_C)
 
 
-def _stream(t) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
-
-
+_stream = _lib.stream_of
 _SM_COUNT = {}
 
 
@@ -175,7 +181,6 @@ def _stage_numel(batch, dim, seqlen, dstate, stage_len):
 
 
 def _register_stage_storage(x, stage_len):
-    from torch.multiprocessing.reductions import StorageWeakRef
     if len(_STAGE_REGISTRY) > 256:
         for key in [k for k, (ref, _) in _STAGE_REGISTRY.items() if ref.expired()]:
             del _STAGE_REGISTRY[key]
@@ -218,27 +223,28 @@ def fwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, delta_softplus, discret
     a, (batch, dim, seqlen, dstate, n_groups, is_complex, var_B, var_C) = _common(
         u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, discretization_method_str)
     n_chunks = (seqlen + CHUNK - 1) // CHUNK
-    with torch.cuda.device(u.device):
+    with _lib.on_device(u):
         out = torch.empty_like(delta)
-        x = torch.empty((batch, dim, n_chunks, dstate * 2), dtype=A.dtype, device=u.device)
         out_z = torch.empty_like(z_) if z_ is not None else None
         a.delta_softplus = int(bool(delta_softplus))
-        a.out, a.x, a.out_z = out.data_ptr(), x.data_ptr(), _ptr(out_z)
-        a.out_bs, a.out_ds = out.stride(0), out.stride(1)
+        a.out, a.out_z = out.data_ptr(), _ptr(out_z)
+        a.out_bs, a.out_ds, _ = out.stride()
         if out_z is not None:
-            a.out_z_bs, a.out_z_ds = out_z.stride(0), out_z.stride(1)
+            a.out_z_bs, a.out_z_ds, _ = out_z.stride()
         S = _segments_for(u, batch, dim, seqlen, dstate, n_groups, is_complex, var_B, var_C, deltaA_,
                           discretization_method_str)
         stage_len = _lib.lib().b200_selscan_stage_states(ctypes.byref(a)) if S <= 1 else 0
+        x_numel = batch * dim * n_chunks * dstate * 2
         if stage_len > 0:
-            x_numel = x.numel()
-            flat = torch.empty(x_numel + _stage_numel(batch, dim, seqlen, dstate, stage_len), dtype=x.dtype,
+            flat = torch.empty(x_numel + _stage_numel(batch, dim, seqlen, dstate, stage_len), dtype=A.dtype,
                                device=u.device)
             x = flat[:x_numel].view(batch, dim, n_chunks, dstate * 2)
             _register_stage_storage(x, stage_len)
-            a.x = x.data_ptr()
-            a.stage_h = x.data_ptr() + x_numel * x.element_size()
+            a.stage_h = flat.data_ptr() + x_numel * 4
             a.stage_len = stage_len
+        else:
+            x = torch.empty((batch, dim, n_chunks, dstate * 2), dtype=A.dtype, device=u.device)
+        a.x = x.data_ptr()
         if S > 1:
             a.l_segments = S
             try:
@@ -271,7 +277,7 @@ def bwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, dout, x_, out_, dz_, de
     _shape(dout, batch, dim, seqlen, name="dout")
     has_z = z_ is not None
     n_chunks = (seqlen + CHUNK - 1) // CHUNK
-    with torch.cuda.device(u.device):
+    with _lib.on_device(u):
         out = dz = out_z = None
         if has_z:
             _check(out_ is not None, "out is required when z is given")
@@ -295,11 +301,19 @@ def bwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, dout, x_, out_, dz_, de
             _shape(x_, batch, dim, n_chunks, 2 * dstate, name="x")
         du = torch.empty_like(u)
         ddelta = torch.empty_like(delta)
-        dA = torch.zeros_like(A)
-        dB = torch.zeros_like(B) if not var_B else torch.zeros_like(B, dtype=torch.float32)
-        dC = torch.zeros_like(C) if not var_C else torch.zeros_like(C, dtype=torch.float32)
-        dD = torch.zeros_like(D_) if D_ is not None else None
-        ddelta_bias = torch.zeros_like(delta_bias_) if delta_bias_ is not None else None
+        if A.is_contiguous() and A.dtype == torch.float32 and var_B and var_C and B.is_contiguous() and C.is_contiguous():
+            # two fills instead of five: the parameters' gradients, and the (larger) sums for B and C
+            n, nD, nb = A.numel(), (0 if D_ is None else dim), (0 if delta_bias_ is None else dim)
+            dA, dD, ddelta_bias = torch.zeros(n + nD + nb, dtype=torch.float32, device=u.device).split((n, nD, nb))
+            dA = dA.view(A.shape)
+            dD, ddelta_bias = (dD if nD else None), (ddelta_bias if nb else None)
+            dB, dC = torch.zeros((2, *B.shape), dtype=torch.float32, device=u.device).unbind(0)
+        else:
+            dA = torch.zeros_like(A)
+            dB = torch.zeros_like(B) if not var_B else torch.zeros_like(B, dtype=torch.float32)
+            dC = torch.zeros_like(C) if not var_C else torch.zeros_like(C, dtype=torch.float32)
+            dD = torch.zeros_like(D_) if D_ is not None else None
+            ddelta_bias = torch.zeros_like(delta_bias_) if delta_bias_ is not None else None
         ddeltaA = torch.empty_like(deltaA_) if deltaA_ is not None else None
 
         q = _lib.struct("b200_selscan_bwd_args")()
@@ -308,11 +322,10 @@ def bwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, dout, x_, out_, dz_, de
         f.stage_h, f.stage_len = _stage_states_of(x_, batch, dim, seqlen, dstate)
         f.out = _ptr(out)
         if out is not None:
-            f.out_bs, f.out_ds = out.stride(0), out.stride(1)
+            f.out_bs, f.out_ds, _ = out.stride()
         f.out_z = _ptr(out_z)
         if out_z is not None:
-            f.out_z_bs, f.out_z_ds = out_z.stride(0), out_z.stride(1)
-        q.f = f
+            f.out_z_bs, f.out_z_ds, _ = out_z.stride()
         q.dout, q.du, q.ddelta = dout.data_ptr(), du.data_ptr(), ddelta.data_ptr()
         q.ddeltaA, q.dz = _ptr(ddeltaA), _ptr(dz)
         q.dA, q.dB, q.dC = dA.data_ptr(), dB.data_ptr(), dC.data_ptr()
@@ -329,23 +342,23 @@ def bwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, dout, x_, out_, dz_, de
                 setattr(q, name, t.data_ptr())
             if h_in is not None:
                 f.stage_h, f.stage_len = None, 0      # stage states of a zero-start forward do not apply
-                q.f = f
-        q.dout_bs, q.dout_ds = dout.stride(0), dout.stride(1)
-        q.du_bs, q.du_ds = du.stride(0), du.stride(1)
-        q.ddelta_bs, q.ddelta_ds = ddelta.stride(0), ddelta.stride(1)
+        q.dout_bs, q.dout_ds, _ = dout.stride()
+        q.du_bs, q.du_ds, _ = du.stride()
+        q.ddelta_bs, q.ddelta_ds, _ = ddelta.stride()
         if ddeltaA is not None:
-            q.ddeltaA_bs, q.ddeltaA_ds = ddeltaA.stride(0), ddeltaA.stride(1)
+            q.ddeltaA_bs, q.ddeltaA_ds, _ = ddeltaA.stride()
         if dz is not None:
-            q.dz_bs, q.dz_ds = dz.stride(0), dz.stride(1)
-        q.dA_ds, q.dA_ns = dA.stride(0), dA.stride(1)
+            q.dz_bs, q.dz_ds, _ = dz.stride()
+        q.dA_ds, q.dA_ns = dA.stride()
         if var_B:
-            q.dB_bs, q.dB_gs, q.dB_ns = dB.stride(0), dB.stride(1), dB.stride(2)
+            q.dB_bs, q.dB_gs, q.dB_ns, _ = dB.stride()
         else:
             q.dB_bs, q.dB_gs, q.dB_ns = 0, dB.stride(0), dB.stride(1)
         if var_C:
-            q.dC_bs, q.dC_gs, q.dC_ns = dC.stride(0), dC.stride(1), dC.stride(2)
+            q.dC_bs, q.dC_gs, q.dC_ns, _ = dC.stride()
         else:
             q.dC_bs, q.dC_gs, q.dC_ns = 0, dC.stride(0), dC.stride(1)
+        q.f = f
         work_bytes = _lib.lib().b200_selscan_bwd_work_bytes(ctypes.byref(q))
         if work_bytes > 0:
             work = torch.empty(work_bytes, dtype=torch.uint8, device=u.device)

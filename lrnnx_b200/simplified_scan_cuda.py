@@ -57,14 +57,14 @@ def _common(u, delta, A, B, C, deltaA, discretization):
 
 
 def _stream(t) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _lib.stream_of(t)
 
 
 def fwd(u, delta, A, B, C, deltaA_, discretization_method_str):
     """Returns ``[out, x]``: out complex64 like u, x (batch, dim, n_chunks, 2*dstate) complex64."""
     a, (batch, dim, seqlen, dstate) = _common(u, delta, A, B, C, deltaA_, discretization_method_str)
     n_chunks = (seqlen + CHUNK - 1) // CHUNK
-    with torch.cuda.device(u.device):
+    with _lib.on_device(u):
         out = torch.empty_like(u)
         x = torch.empty((batch, dim, n_chunks, 2 * dstate), dtype=torch.complex64, device=u.device)
         a.out, a.x = out.data_ptr(), x.data_ptr()
@@ -90,7 +90,7 @@ def bwd(u, delta, A, B, C, deltaA_, dout, x_, discretization_method_str, need_dB
         _check(x_.dtype == torch.complex64 and x_.is_cuda and x_.is_contiguous(),
                "x must be a contiguous complex64 CUDA tensor")
         _check(tuple(x_.shape) == (batch, dim, n_chunks, 2 * dstate), "x has the wrong shape")
-    with torch.cuda.device(u.device):
+    with _lib.on_device(u):
         du = torch.empty_like(u)
         ddelta = torch.empty_like(delta)
         if A.is_contiguous() and B.is_contiguous() and C.is_contiguous():

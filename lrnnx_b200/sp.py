@@ -74,8 +74,8 @@ def apply_fixup(u, delta, A, B, C, D, z, delta_bias, delta_softplus, out, x, out
     p_in = p_in.float().contiguous()
     q.h_in, q.p_in = h_in.data_ptr(), p_in.data_ptr()
     q.n_segments, q.seg_len = 0, 0
-    with torch.cuda.device(u.device):
-        _lib.call("b200_selscan_fixup", q, torch.cuda.current_stream(u.device).cuda_stream)
+    with _lib.on_device(u):
+        _lib.call("b200_selscan_fixup", q, _lib.stream_of(u))
 
 
 def adjoint_summary(delta, A, C, z, delta_bias, delta_softplus, dout, discretization="mamba"):
@@ -87,11 +87,11 @@ def adjoint_summary(delta, A, C, z, delta_bias, delta_softplus, dout, discretiza
     a.delta_softplus = int(bool(delta_softplus))
     q = _lib.struct("b200_selscan_adjsum_args")()
     q.f = a
-    with torch.cuda.device(delta.device):
+    with _lib.on_device(delta):
         G = torch.empty(batch, dim, dstate, dtype=torch.float32, device=delta.device)
         q.dout, q.G = dout.data_ptr(), G.data_ptr()
         q.dout_bs, q.dout_ds = dout.stride(0), dout.stride(1)
-        _lib.call("b200_selscan_adjoint_summary", q, torch.cuda.current_stream(delta.device).cuda_stream)
+        _lib.call("b200_selscan_adjoint_summary", q, _lib.stream_of(delta))
     return G
 
 

@@ -17,7 +17,7 @@ def _check(cond: bool, msg: str) -> None:
 
 
 def _stream(t) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _lib.stream_of(t)
 
 
 def _args(v, z, w, seqlen):
@@ -48,7 +48,7 @@ def cauchy_mult_sym_fwd(v, z, w):
     batch, n = v.shape
     L = z.size(0)
     v, z, w = _c64("v", v, batch, n), _c64("z", z, L), _c64("w", w, batch, n)
-    with torch.cuda.device(v.device):
+    with _lib.on_device(v):
         out = torch.empty((batch, L), dtype=v.dtype, device=v.device)
         a = _args(v, z, w, L)
         a.out = out.data_ptr()
@@ -62,7 +62,7 @@ def cauchy_mult_sym_bwd(v, z, w, dout):
     L = z.size(0)
     v, z, w = _c64("v", v, batch, n), _c64("z", z, L), _c64("w", w, batch, n)
     dout = _c64("dout", dout, batch, L)
-    with torch.cuda.device(v.device):
+    with _lib.on_device(v):
         dv, dw = torch.empty_like(v), torch.empty_like(w)
         a = _args(v, z, w, L)
         a.dout, a.dv, a.dw = dout.data_ptr(), dv.data_ptr(), dw.data_ptr()
@@ -78,7 +78,7 @@ def vand_log_mult_sym_fwd(v, x, L):
     batch, n = v.shape
     v, x = _c64("v", v, batch, n), _c64("x", x, batch, n)
     L = int(L)
-    with torch.cuda.device(v.device):
+    with _lib.on_device(v):
         out = torch.empty((batch, L), dtype=torch.float32, device=v.device)
         a = _args(v, None, x, L)
         a.out = out.data_ptr()
@@ -94,7 +94,7 @@ def vand_log_mult_sym_bwd(v, x, dout):
            "dout must be a (batch, L) float32 CUDA tensor")
     dout = dout.contiguous()
     L = dout.size(1)
-    with torch.cuda.device(v.device):
+    with _lib.on_device(v):
         dv, dx = torch.empty_like(v), torch.empty_like(x)
         a = _args(v, None, x, L)
         a.dout, a.dv, a.dw = dout.data_ptr(), dv.data_ptr(), dx.data_ptr()

@@ -426,7 +426,9 @@ int b200_rmsnorm_bwd(const b200_rmsnorm_args *args, void *stream);
  *   w_planes : float32 (4, M, K), K contiguous: Re(W) rounded to TF32 (low 13 mantissa bits
  *              zero), the remainder rounded to TF32, and the same two planes of Im(W)
  *   x        : complex64 (batch, K, N) dense;  out : complex64 (batch, M, N), N contiguous
- * M a multiple of 128, K of 32, N of 64; all pointers 16-byte aligned.
+ * M a multiple of 128, K of 32, N of 64; all pointers 16-byte aligned.  With `padded` the sizes
+ * are free: w_planes is (4, Mp, Kp), Mp and Kp the next multiples of 128 and 32, with zeros in the
+ * padding, the pitches x_ks and x_bs are any even numbers, and out is 8-byte aligned.
  * ------------------------------------------------------------------------ */
 typedef struct b200_cgemm_args {
   int32_t batch, M, K, N;
@@ -434,28 +436,32 @@ typedef struct b200_cgemm_args {
   void *out;
   int64_t x_bs, x_ks;        /* complex elements */
   int64_t out_bs, out_ms;    /* complex elements */
+  int32_t padded, reserved0; /* non-zero: w_planes are padded and the sizes are free */
 } b200_cgemm_args;
 
 int b200_cgemm_wx(const b200_cgemm_args *args, void *stream);
 
 /* Weight gradient of a projection on the tensor cores (same 3xTF32 arithmetic):
  *     out (M x N) += sum over b, l of g[b, m, l] * conj(u[b, n, l])
- * g (batch, M, L), u (batch, N, L), out (M, N): complex64, dense, L contiguous.  out must be
+ * g (batch, M, L), u (batch, N, L), out (M, N): complex64, L contiguous, out dense.  out must be
  * zero-filled by the caller (the contraction is cut over several thread blocks which add their
- * partial results with float32 reductions).  M and N multiples of 128, L of 16. */
+ * partial results with float32 reductions).  Dense operands with M and N multiples
+ * of 128 and L of 16, or any sizes with g_rs, u_rs: row pitches of g and u in elements, even (the
+ * batch entries follow one another: entry b starts b M (b N) rows in). */
 typedef struct b200_cgemm_grad_args {
   int32_t batch, M, N, L;
   const void *g, *u;
   void *out;
+  int64_t g_rs, u_rs;
 } b200_cgemm_grad_args;
 
 int b200_cgemm_grad(const b200_cgemm_grad_args *args, void *stream);
 
 /* Builds the w_planes operand of b200_cgemm_wx from a complex64 matrix W (M, K) given by element
  * strides (so a transposed view is free), optionally conjugated (conj != 0): planes is float32
- * (4, M, K), written densely. */
+ * (4, M, K), written densely, or (padded != 0) (4, Mp, Kp) as above. */
 typedef struct b200_cgemm_planes_args {
-  int32_t M, K, conj, reserved0;
+  int32_t M, K, conj, padded;
   const void *w;
   void *planes;
   int64_t w_rs, w_cs;        /* complex elements */

@@ -21,19 +21,24 @@ from . import projection
 _VALID = ("bilinear", "zoh", "dirac")
 
 
-def _proj(W, x, conj_transpose=False):
-    """W x (or W^H x) per batch: the tensor-core kernel where its tiling applies, einsum otherwise."""
+def _proj(W, x, conj_transpose=False, padded=False):
+    """W x (or W^H x) per batch: the tensor-core kernel, or an einsum for very small products."""
     Wm = W.conj().transpose(0, 1) if conj_transpose else W
-    if projection.supported(Wm, x if x.is_contiguous() else x.contiguous()):
-        return projection.project(W, x, conj_transpose)
+    if projection.fits(Wm, x):
+        return projection.product(W, x, conj_transpose, padded)
     return torch.einsum("mk,bkn->bmn", Wm, x)
 
 
 def _wgrad(g, u):
-    """sum over batch and time of g u^H: the tensor-core kernel where its tiling applies, einsum otherwise."""
-    if projection.grad_supported(g, u):
-        return projection.weight_grad(g, u)
+    """sum over batch and time of g u^H: the tensor-core kernel, or an einsum for very small products."""
+    if projection.grad_fits(g, u):
+        return projection.gradient(g, u)
     return torch.einsum("bml,bnl->mn", g, u.conj())
+
+
+def _rows(x, W):
+    """x with rows that the projection kernels read in place, where they will be used with W."""
+    return projection.rows(x) if x.is_complex() and projection.fits(W, x) else x
 
 
 def _kernel_A(A):
@@ -52,7 +57,7 @@ class SimplifiedScanFn(torch.autograd.Function):
         P = A.shape[0]
         A_k = _kernel_A(A).contiguous()
         dstate = A_k.shape[1]
-        Bu = _proj(B, u)
+        Bu = _proj(B, u, padded=True)
         ident = torch.ones(P, dstate, dtype=A.dtype, device=A.device)
         out, xs = simplified_scan_cuda.fwd(Bu, delta, A_k, ident, ident, deltaA, discretization)
         y = _proj(C, out)
@@ -68,7 +73,8 @@ class SimplifiedScanFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout, *args):
         u, delta, A_k, B, C, Bu, out, xs, ident, deltaA = ctx.saved_tensors
-        dx_out = _proj(C, dout, conj_transpose=True)
+        dout, u = _rows(dout, C.t()), _rows(u, B)
+        dx_out = _proj(C, dout, conj_transpose=True, padded=True)
         dC = _wgrad(dout, out)
         if dx_out.stride(-1) != 1:
             dx_out = dx_out.contiguous()
@@ -103,7 +109,7 @@ class S5InnerFn(torch.autograd.Function):
         P = A.shape[0]
         A_k = _kernel_A(A).contiguous()
         dstate = A_k.shape[1]
-        Bu = _proj(B, u)
+        Bu = _proj(B, u, padded=True)
         ident = torch.ones(P, dstate, dtype=A.dtype, device=A.device)
         scan_out, xs = simplified_scan_cuda.fwd(Bu, delta, A_k, ident, ident, deltaA, discretization)
         y_complex = _proj(C, scan_out)
@@ -124,7 +130,8 @@ class S5InnerFn(torch.autograd.Function):
         du_skip = D.unsqueeze(0).unsqueeze(-1) * dout
         scale = 2.0 if ctx.conj_sym else 1.0
         dy_complex = torch.complex(scale * dout, torch.zeros_like(dout))
-        dscan = _proj(C, dy_complex, conj_transpose=True)
+        dy_complex, u = _rows(dy_complex, C.t()), _rows(u, B)
+        dscan = _proj(C, dy_complex, conj_transpose=True, padded=True)
         dC = _wgrad(dy_complex, scan_out)
         if dscan.stride(-1) != 1:
             dscan = dscan.contiguous()

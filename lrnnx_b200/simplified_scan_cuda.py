@@ -60,12 +60,20 @@ def _stream(t) -> int:
     return _lib.stream_of(t)
 
 
+def _like(u):
+    """An output for u: with u's rows where they are padded to an even pitch, dense otherwise."""
+    L = u.shape[2]
+    if u.stride() == (u.shape[1] * (L + 1), L + 1, 1):
+        return torch.empty_strided(u.shape, u.stride(), dtype=u.dtype, device=u.device)
+    return torch.empty_like(u)
+
+
 def fwd(u, delta, A, B, C, deltaA_, discretization_method_str):
     """Returns ``[out, x]``: out complex64 like u, x (batch, dim, n_chunks, 2*dstate) complex64."""
     a, (batch, dim, seqlen, dstate) = _common(u, delta, A, B, C, deltaA_, discretization_method_str)
     n_chunks = (seqlen + CHUNK - 1) // CHUNK
     with _lib.on_device(u):
-        out = torch.empty_like(u)
+        out = _like(u)
         x = torch.empty((batch, dim, n_chunks, 2 * dstate), dtype=torch.complex64, device=u.device)
         a.out, a.x = out.data_ptr(), x.data_ptr()
         a.out_bs, a.out_ds = out.stride(0), out.stride(1)
@@ -91,7 +99,7 @@ def bwd(u, delta, A, B, C, deltaA_, dout, x_, discretization_method_str, need_dB
                "x must be a contiguous complex64 CUDA tensor")
         _check(tuple(x_.shape) == (batch, dim, n_chunks, 2 * dstate), "x has the wrong shape")
     with _lib.on_device(u):
-        du = torch.empty_like(u)
+        du = _like(u)
         ddelta = torch.empty_like(delta)
         if A.is_contiguous() and B.is_contiguous() and C.is_contiguous():
             dA, dB, dC = torch.zeros((3,) + tuple(A.shape), dtype=A.dtype, device=A.device).unbind(0)  # one fill

@@ -1,0 +1,70 @@
+"""The tensor-core projections at sizes that are no multiple of their tiles (128 weight rows, 32 and 16 floats of K,
+64 complex columns), odd lengths and padded rows, against float64.  Bound: the products are rounded to about
+2^-21 each, the sums to 2^-23 of a chain of 32; 1e-6 of the largest output is a few times what both give."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _cn(g, *shape):
+    return torch.complex(torch.randn(*shape, generator=g), torch.randn(*shape, generator=g)).cuda()
+
+
+def _close(got, want):
+    from lrnnx_b200 import _lib
+    torch.cuda.synchronize()
+    assert _lib.lib().b200_device_status() == 0
+    assert got.shape == want.shape
+    assert float((got.to(torch.complex128) - want).abs().max()) <= 1e-6 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("M,K,N", [(32, 32, 1), (33, 47, 63), (128, 49, 64), (129, 32, 65), (200, 130, 257), (256, 512, 129)])
+@pytest.mark.parametrize("conj", [False, True])
+def test_product(M, K, N, conj):
+    from lrnnx_b200.ops import projection
+    g = torch.Generator().manual_seed(M + K + N)
+    W, x = _cn(g, *((K, M) if conj else (M, K))), _cn(g, 3, K, N)
+    want = torch.einsum("mk,bkn->bmn", (W.mH if conj else W).to(torch.complex128), x.to(torch.complex128))
+    assert projection.fits(W.mH if conj else W, x)
+    _close(projection.product(W, x, conj), want)
+    padded = projection.product(W, x, conj, padded=True)
+    assert padded.stride(1) % 2 == 0
+    _close(padded, want)
+    _close(projection.product(W.conj().resolve_conj(), torch.cat([x, x], 2)[..., :N], conj).conj(),
+           torch.einsum("mk,bkn->bmn", (W.mH if conj else W).to(torch.complex128), x.conj().to(torch.complex128)))
+
+
+@pytest.mark.parametrize("M,N,L", [(32, 33, 1), (40, 129, 7), (128, 128, 9), (130, 64, 255), (257, 200, 1999)])
+def test_gradient(M, N, L):
+    from lrnnx_b200.ops import projection
+    g = torch.Generator().manual_seed(M + N + L)
+    a, b = _cn(g, 3, M, L), _cn(g, 3, N, L)
+    want = torch.einsum("bml,bnl->mn", a.to(torch.complex128), b.to(torch.complex128).conj())
+    assert projection.grad_fits(a, b)
+    _close(projection.gradient(a, b), want)
+    _close(projection.gradient(projection.rows(a), projection.rows(b)), want)
+
+
+@pytest.mark.parametrize("L", [63, 64, 2049])
+def test_simplified_scan_at_odd_lengths(L):
+    """Intermediate results in padded rows: output and gradients agree with the einsum formulation on the same scan kernels."""
+    from lrnnx_b200.ops import simplified_scan_fn
+    from oracle import scan_oracle as O
+    g = torch.Generator().manual_seed(L)
+    P, H = 48, 40
+    A = torch.complex(-0.05 - 0.1 * torch.rand(P, generator=g), torch.rand(P, generator=g))
+    t = [_cn(g, 2, H, L).cpu(), 0.5 + torch.rand(2, P, L, generator=g), A, _cn(g, P, H).cpu() / H ** 0.5, _cn(g, H, P).cpu() / P ** 0.5]
+    gout = _cn(g, 2, H, L).cpu()
+
+    def run(fn, cast, **kw):
+        leaves = [cast(v).requires_grad_(True) for v in t]
+        y = fn(*leaves, discretization="zoh", **kw)
+        return [y.detach().cpu()] + [v.cpu() for v in torch.autograd.grad(y, leaves, cast(gout))]
+
+    wide = lambda v: v.to(torch.complex128 if v.is_complex() else torch.float64)  # noqa: E731
+    want = run(O.simplified_scan_oracle, wide, compute_dtype=torch.float64)
+    for a, b in zip(run(simplified_scan_fn, lambda v: v.cuda()), want):
+        assert float((wide(a) - b).abs().max()) <= 1e-5 * float(b.abs().max())

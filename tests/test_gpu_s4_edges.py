@@ -1,0 +1,45 @@
+"""Cauchy kernels at the edges of their tiles: positions go in packed pairs (128 apart in the forward, 256 in the
+backward, 512 to a thread block), poles in tiles of 4 and in shared-memory blocks of 1024."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -24
+
+
+def _case(rows, n, length):
+    g = torch.Generator().manual_seed(rows * 7919 + n * 131 + length)
+    r = lambda *s: torch.randn(*s, generator=g)
+    v = torch.complex(r(rows, n), r(rows, n))
+    w = torch.complex(-0.01 - r(rows, n).abs(), 3 * r(rows, n))
+    z = torch.complex(0.05 + 0.05 * r(length).abs(), 4 * r(length))
+    return v, z, w, torch.complex(r(rows, length), r(rows, length))
+
+
+@pytest.mark.parametrize("rows,n,length", [(1, 1, 1), (3, 5, 127), (2, 4, 129), (2, 3, 255), (3, 2, 257), (2, 7, 384),
+                                           (1, 33, 511), (2, 32, 512), (3, 6, 513), (1, 1025, 641), (2, 9, 1025),
+                                           (1, 2, 4099)])
+def test_cauchy_at_tile_edges(rows, n, length):
+    from lrnnx_b200.ops import cauchy_mult
+    v, z, w, g = _case(rows, n, length)
+    vg, wg = v.cuda().requires_grad_(True), w.cuda().requires_grad_(True)
+    out = cauchy_mult(vg, z.cuda(), wg)
+    dv, dw = torch.autograd.grad(out, (vg, wg), g.cuda())
+    V, Z, W, G = (t.to(torch.cdouble) for t in (v, z, w, g))
+    k1, k2 = 1 / (Z - W[..., None]), 1 / (Z - W[..., None].conj())              # (rows, n, length)
+    V, G = V[..., None], G[:, None]
+    # A term is exact up to the roundings of its factors: 1 for each of dr, e1, e2 and 3 for the squared modulus,
+    # which enter it once or twice, 2 for the reciprocal and 3 for the products: at most 16, twice that with a
+    # squared reciprocal.  Adding up m terms in any order costs m roundings of the sum of the moduli.
+    want = {"out": (V * k1 + V.conj() * k2).sum(1), "dv": (G * k1.conj() + G.conj() * k2).sum(2),
+            "dw": (V.conj() * (G * k1.conj() ** 2 + G.conj() * k2 ** 2)).sum(2)}
+    size = {"out": (V.abs() * (k1.abs() + k2.abs())).sum(1), "dv": (G.abs() * (k1.abs() + k2.abs())).sum(2),
+            "dw": (V.abs() * G.abs() * (k1.abs() ** 2 + k2.abs() ** 2)).sum(2)}
+    # per-thread chains (2 terms per pole; 2 per 256 positions of a chunk), then 5 + 8 sums over lanes and warps and
+    # the chunks (at least 1024 positions each)
+    chain = length // 128 + 16 + length // 1024
+    steps = {"out": 16 + 4 * n, "dv": 16 + chain, "dw": 36 + chain}
+    for name, got in (("out", out.detach()), ("dv", dv), ("dw", dw)):
+        err = (got.cpu().to(torch.cdouble) - want[name]).abs()
+        bad = err > 2 * steps[name] * EPS * size[name]
+        assert not bool(bad.any()), f"{name}: {int(bad.sum())} values outside, worst {float((err / size[name]).max()):.2e}"

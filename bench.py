@@ -125,8 +125,6 @@ class ClockSampler:
 NCU_TRAFFIC = {
     ("s5_scan_cfg1", "simpscan_fwd_kernel"): 127.6e6,
     ("s5_scan_cfg1", "simpscan_bwd_kernel"): 301.5e6,
-    ("s6_layer_cfg2", "selscan_fwd"): 223.4e6,
-    ("s6_layer_cfg2", "selscan_bwd"): 382.2e6,
     ("cauchy_s4", "cauchy_fwd"): 76.1e6,
 }
 

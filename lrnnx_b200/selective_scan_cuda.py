@@ -135,11 +135,11 @@ _stream = _lib.stream_of
 _SM_COUNT = {}
 
 
-def _segments_for(u, batch, dim, seqlen, dstate, n_groups, is_complex, var_B, var_C, deltaA, method):
+def _segments_for(u, batch, dim, seqlen, dstate, n_groups, is_complex, var_B, var_C, deltaA, method, rows=()):
     """Number of sequence segments for the forward call: > 1 only for long rows that would leave
     part of the GPU idle, on the shape class of the state-parallel kernels.  Segments are scanned
     concurrently from zero states and stitched by the summary fold + fix-up that the multi-GPU
-    sequence-parallel path uses."""
+    sequence-parallel path uses.  ``rows``: the call's (batch, ..., L) operands."""
     if is_complex or method != "mamba" or not (var_B and var_C) or deltaA is not None or dstate != 16:
         return 1
     if seqlen < 4 * CHUNK:
@@ -148,7 +148,12 @@ def _segments_for(u, batch, dim, seqlen, dstate, n_groups, is_complex, var_B, va
     if idx not in _SM_COUNT:
         _SM_COUNT[idx] = torch.cuda.get_device_properties(idx).multi_processor_count
     sms = _SM_COUNT[idx]
-    rows = batch * dim
+    if u.dtype != torch.float32:
+        # 16-bit outputs behind a cut are rounded twice, by the segment and by the fix-up: the places of the cuts show
+        # in the results, and calls without cuts are the more exact.  So only what has always been cut is (whole
+        # tiles of 16 channels and 8 steps, in whole 16-byte pieces of rows), and where it has always been.
+        return _segments_16bit(batch * dim // 16, seqlen, 8 * sms) if _whole_tiles(dim // n_groups, seqlen, rows) else 1
+    n_rows = batch * dim
     ctas = batch * n_groups * -(-(dim // n_groups) // 32)       # thread blocks of 32 channels; 3 fit on an SM
     if ctas >= 12 * sms:
         return 1
@@ -156,15 +161,38 @@ def _segments_for(u, batch, dim, seqlen, dstate, n_groups, is_complex, var_B, va
     # the fix-up of a segment takes 6 ns per row
     step_ns = (0, 60, 80, 105)
     best, best_ns = 1, None
+    for S, seg_len in _cuts(seqlen):
+        full, rest = divmod(ctas * S, 3 * sms)
+        ns = (full * step_ns[3] + step_ns[-(-rest // sms)]) * seg_len + 6 * n_rows * (S - 1)
+        if best_ns is None or ns < 0.95 * best_ns:
+            best, best_ns = S, ns
+    return best
+
+
+def _cuts(seqlen):
+    """Segment counts up to 16, and the segments' length: whole checkpoint chunks, two at least."""
     for want in range(1, 17):
         seg_len = -(-(-(-seqlen // want)) // CHUNK) * CHUNK
         if want > 1 and seg_len < 2 * CHUNK:
-            break
-        S = -(-seqlen // seg_len)
-        full, rest = divmod(ctas * S, 3 * sms)
-        ns = (full * step_ns[3] + step_ns[-(-rest // sms)]) * seg_len + 6 * rows * (S - 1)
-        if best_ns is None or ns < 0.95 * best_ns:
-            best, best_ns = S, ns
+            return
+        yield -(-seqlen // seg_len), seg_len
+
+
+def _whole_tiles(channels, seqlen, rows):
+    return channels % 16 == 0 and seqlen % 8 == 0 and all(
+        t is None or (t.data_ptr() % 16 == 0 and all(s % 8 == 0 for s in t.stride()[:-1])) for t in rows)
+
+
+def _segments_16bit(tiles, seqlen, slots):
+    """The segment count whose ``tiles`` (16 channels each) fill whole waves of ``slots`` best; ties: fewer segments."""
+    if tiles >= 4 * slots:
+        return 1
+    best, best_eff = 1, 0.0
+    for S, _ in _cuts(seqlen):
+        waves = tiles * S / slots
+        eff = waves if waves <= 1.0 else waves / -(-waves // 1)
+        if eff > best_eff * 1.10 + 1e-9:
+            best, best_eff = S, eff
     return best
 
 
@@ -232,7 +260,7 @@ def fwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, delta_softplus, discret
         if out_z is not None:
             a.out_z_bs, a.out_z_ds, _ = out_z.stride()
         S = _segments_for(u, batch, dim, seqlen, dstate, n_groups, is_complex, var_B, var_C, deltaA_,
-                          discretization_method_str)
+                          discretization_method_str, (u, delta, B, C, z_, out, out_z))
         stage_len = _lib.lib().b200_selscan_stage_states(ctypes.byref(a)) if S <= 1 else 0
         x_numel = batch * dim * n_chunks * dstate * 2
         if stage_len > 0:

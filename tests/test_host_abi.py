@@ -119,3 +119,27 @@ def test_every_python_module_of_the_package_imports():
         if mod.name.endswith(".build"):
             continue
         importlib.import_module(mod.name)
+
+
+def test_16bit_calls_are_cut_where_they_always_were(monkeypatch):
+    """16-bit results depend on where a long sequence is cut, because they are rounded once more behind a cut: the cuts of
+    whole tiles stay where they were, and other calls stay in one piece."""
+    from lrnnx_b200 import selective_scan_cuda as ext
+    monkeypatch.setitem(ext._SM_COUNT, 0, 148)
+
+    class U:
+        device = torch.device("cuda:0")
+
+    def cuts(dtype, batch, dim, L, groups=1, rows=()):
+        U.dtype = dtype
+        return ext._segments_for(U, batch, dim, L, 16, groups, False, True, True, None, "mamba", rows)
+
+    for dtype in (torch.bfloat16, torch.float16):
+        for shape, want in (((1, 5120, 131072), 7), ((1, 16, 10504), 3), ((1, 512, 32768), 8), ((2, 1024, 16384), 4), ((8, 1536, 16384), 3),
+                            ((1, 5120, 8184), 1), ((64, 4096, 8192), 1), ((1, 4096, 65536), 4), ((4, 4736, 32768), 1)):
+            assert cuts(dtype, *shape) == want, shape
+        assert cuts(dtype, 1, 512, 32767) == cuts(dtype, 1, 520, 32768) == cuts(dtype, 1, 512, 32768, groups=64) == 1
+        rows = torch.zeros(1, 8, 40, dtype=dtype)
+        assert cuts(dtype, 1, 512, 32768, rows=(rows, None)) == 8
+        assert cuts(dtype, 1, 512, 32768, rows=(rows[..., 1:],)) == cuts(dtype, 1, 512, 32768, rows=(rows[..., :39].contiguous(),)) == 1
+    assert cuts(torch.float32, 1, 512, 32767) > 1

@@ -10,7 +10,8 @@
 // runs the adjoint in the same pass: g_t = dy_t B C + q_t, q_{t-1} = a_t g_t.
 // Measured, 4 x 1024 rows x 2048 steps: forward 29 us, backward 59 us (the one-warp-per-row coverage kernels: 151 and
 // 378 us; the bytes alone: 15 and 25 us at the copy rate).
-// The RG-LRU input gain sqrt(1 - a^2) is taken from expm1, which keeps it exact where a is close to 1.
+// The RG-LRU input gain sqrt(1 - a^2) is taken from expm1, which keeps it exact where a is close to 1; the transition
+// itself is the exponential where it is small (dA is divided by A, so a's error counts relative to a).
 #include "common.cuh"
 #include "dispatch.h"
 
@@ -49,22 +50,24 @@ __device__ __forceinline__ void store(float *row, int t0, int L, float *buf, int
   __syncwarp();
 }
 
-// exp(x) - 1: its Taylor series to x^10 for |x| <= 1 (truncation below 3e-8 of the result), the SFU's exponential
-// elsewhere (x < -1: no cancellation is left)
-__device__ __forceinline__ float expm1_(float x) {
-  float e;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * kLog2e));
+// e = exp(x) and m = exp(x) - 1, each accurate relative to itself.  For |x| <= 1 m is the Taylor series to x^10
+// (truncation below 4e-8 of m) and e = 1 + m, at least 0.36, loses half a unit of 1.  Elsewhere nothing cancels in
+// m = e - 1, but 1 + m would keep only e's bits above 2^-24: there e itself is the exponential.
+__device__ __forceinline__ void exp_expm1(float x, float &e, float &m) {
+  const float big = expf(x);
   float s = fmaf(x, 1.f / 10.f, 1.f);
 #pragma unroll
   for (int k = 9; k >= 2; --k) s = fmaf(x * (1.f / k), s, 1.f);
-  return fabsf(x) <= 1.f ? x * s : e - 1.f;
+  const bool near0 = fabsf(x) <= 1.f;
+  m = near0 ? x * s : big - 1.f;
+  e = near0 ? 1.f + m : big;
 }
 
 // transition a, input gain k
 template <int DM> __device__ __forceinline__ void coef(float logA, float d, float &a, float &k) {
   if constexpr (DM == B200_DISC_RGLRU) {          // a = A^d, k = sqrt(1 - a^2)
-    const float m = expm1_(d * logA);
-    a = 1.f + m;
+    float m;
+    exp_expm1(d * logA, a, m);
     k = sqrtf(-m * (2.f + m));
   } else {                                        // S7: a = 1 - 1 / (d^2 + 1/2), k = 1
     a = 1.f - 1.f / (d * d + 0.5f);

@@ -34,3 +34,27 @@ def test_one_state_rows(method, L):
     # a product of up to a few hundred factors near 1, each with a rounding of 6e-8: 1e-4 leaves room for all of them
     for name, a, b in zip(["out", "last"] + ["d" + n for n in names], got, want):
         assert_close(a, b.float(), rtol=1e-4, atol_scale=2e-5, name=name)
+
+
+@pytest.mark.parametrize("delta", [0.5, 1.0, 8.0])
+def test_rglru_strong_decay(delta):
+    """Transitions A**delta down to 1e-30, every row on its own scale (a row has one A).  Bound: a is exact relative to
+    itself up to the rounding of x = delta log A, |x| 2^-24 <= 4e-6, and a few roundings of 6e-8; twice that.  u and
+    dout are positive, so the sums that make dA do not cancel."""
+    from lrnnx_b200.ops import rglru_scan_fn
+    g = torch.Generator().manual_seed(7)
+    A = torch.tensor([0.5, 0.3, 0.1, 0.05, 1e-2, 1e-3, 1e-4, 1e-6, 1e-7, 1e-8])
+    A = A[A.double() ** (1.1 * delta) > 1e-30].unsqueeze(-1)
+    shape = (2, A.shape[0], 300)
+    u, dout = (0.75 + 0.5 * torch.rand(shape, generator=g) for _ in range(2))
+    d = delta * (1 + 0.1 * torch.rand(shape, generator=g))
+
+    def run(fn, cast, **kw):
+        leaves = [cast(v).requires_grad_(True) for v in (u, d, A)]
+        out = fn(*leaves, **kw)
+        return [out.detach().cpu().double()] + [x.cpu().double() for x in torch.autograd.grad(out, leaves, cast(dout))]
+
+    want = run(O.rglru_scan_oracle, lambda v: v.double(), compute_dtype=torch.float64)
+    for name, a, b in zip(("out", "du", "ddelta", "dA"), run(rglru_scan_fn, lambda v: v.cuda()), want):
+        err = (a - b).abs().amax(-1) / b.abs().amax(-1)
+        assert float(err.max()) <= 1e-5, f"{name}: error by rows {err.tolist()}"

@@ -74,7 +74,7 @@ int b200_selscan_fwd(const b200_selscan_fwd_args *args, void *stream) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (selscan_seq_supported(*args)) {
     b200_selscan_fwd_args a = *args;
-    if (a.stage_len <= 0 || a.stage_len % kStageUnit) a.stage_h = nullptr;     // stage states come in whole stages of the kernel
+    if (!stage_usable(a.stage_len)) a.stage_h = nullptr;
     return selscan_seq_fwd(a, st);
   }
   B200_REQUIRE(args->l_segments <= 1, B200_ERR_UNSUPPORTED,
@@ -114,7 +114,8 @@ int b200_selscan_bwd(const b200_selscan_bwd_args *args, void *stream) {
   if (!args->h_in && !args->q_in && selscan_row1_supported(f)) return selscan_row1_bwd(*args, st);
   if (!selscan_seq_bwd_supported(*args)) return selscan_bwd_generic(*args, st);
   b200_selscan_bwd_args a = *args;
-  if (a.f.stage_len <= 0 || kChunk % a.f.stage_len || a.f.stage_len % kStageUnit) a.f.stage_h = nullptr;
+  if (!stage_usable(a.f.stage_len)) a.f.stage_h = nullptr;
+  B200_REQUIRE((reinterpret_cast<uintptr_t>(a.work) & 31) == 0, B200_ERR_ALIGN, "selscan_bwd: work must be 32-byte aligned");
   if (a.work) return selscan_seq_bwd(a, a.work, a.work_bytes, st);
   void *work = nullptr;
   const int64_t bytes = selscan_seq_bwd_bytes(f);

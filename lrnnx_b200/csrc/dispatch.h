@@ -5,7 +5,10 @@
 
 namespace b200 {
 
-constexpr int kStageUnit = 32;    // stage_h spacings of the state-parallel kernels are multiples of this
+constexpr int kStage = 256;       // the state-parallel backward starts its walks every so many steps
+// Spacings of stage_h that it can start them from: whole 32-step stages, of which one ends where each walk begins.
+// States of any other spacing are neither written nor read.
+inline bool stage_usable(int stage_len) { return stage_len > 0 && stage_len % 32 == 0 && kStage % stage_len == 0; }
 
 // coverage kernels: every variant (selscan_generic.cu)
 int selscan_fwd_generic(const b200_selscan_fwd_args &a, cudaStream_t st);

@@ -320,7 +320,7 @@ bool selscan_seq_supported(const b200_selscan_fwd_args &a) {
 int selscan_seq_stage_len(const b200_selscan_fwd_args &a) {
   const char *e = getenv("LRNNX_B200_SL_MIN_WARPS");
   const int64_t warps = (int64_t)a.batch * ((a.dim + 15) / 16);
-  return e && warps >= atoll(e) ? 32 : 256;
+  return e && warps >= atoll(e) ? 32 : kStage;
 }
 
 int selscan_seq_fwd(const b200_selscan_fwd_args &a, cudaStream_t st) {

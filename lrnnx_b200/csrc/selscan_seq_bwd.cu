@@ -604,7 +604,7 @@ template <typename T> int launch_bwd(const b200_selscan_bwd_args &a, float4 *hs,
   SeqPre x{};
   x.hs = hs;
   x.qs = qs;
-  x.piece = f.stage_h ? 256 : kChunk;
+  x.piece = f.stage_h ? kStage : kChunk;
   x.tiles = f.n_groups * ((cpg + FW * QCH - 1) / (FW * QCH));
   x.adj = f.batch * x.tiles;
   const bool al = row16<T>(f.u, f.u_bs, f.u_ds) && row16<T>(f.delta, f.delta_bs, f.delta_ds) && row16<T>(a.dout, a.dout_bs, a.dout_ds) &&
@@ -662,7 +662,7 @@ bool selscan_seq_bwd_supported(const b200_selscan_bwd_args &a) {
     if (ds * 4 != (int32_t)(ds * 4)) return false;          // row pitches in bytes are 32-bit numbers in the kernel
   const int64_t cpg = a.f.dim / a.f.n_groups;
   const int64_t gx = (int64_t)a.f.batch * a.f.n_groups * ((a.f.seqlen + BT - 1) / BT);
-  const int64_t pre = (int64_t)a.f.batch * a.f.n_groups * ((cpg + FW * QCH - 1) / (FW * QCH)) * (1 + (a.f.seqlen + 255) / 256);
+  const int64_t pre = (int64_t)a.f.batch * a.f.n_groups * ((cpg + FW * QCH - 1) / (FW * QCH)) * (1 + (a.f.seqlen + kStage - 1) / kStage);
   return (al & 15) == 0 && gx < (int64_t)1 << 31 && pre < (int64_t)1 << 31;
 }
 

@@ -89,3 +89,35 @@ def test_backward_workspaces(L, monkeypatch):
         got = ext.bwd(*args, dout, x.clone() if mode == "checkpoints" else x, out, None, True, False, "mamba")
         for i, (a, b) in enumerate(zip(got, want)):
             assert_close(a.cpu(), b.cpu(), rtol=2e-5, atol_scale=2e-6, name=f"{mode} gradient {i}")
+
+
+@pytest.mark.parametrize("stage_len", [512, 1024, 2048, 96])
+def test_stage_states_of_another_spacing(stage_len, monkeypatch):
+    """A caller of the C entry points that keeps its stage states at a spacing other than the one it was told: the
+    backward, which starts walks every 256 steps, recomputes them instead of reading past the ones that are there."""
+    from lrnnx_b200 import _lib
+    from lrnnx_b200 import selective_scan_cuda as ext
+    t, g = _make_inputs(1, 24, 16, 2500, seed=1)
+    c = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in t.items()}
+    args = (c["u"], c["delta"], c["A"], c["B"], c["C"], c["D"], c["z"], c["delta_bias"], None)
+    out, x, _ = ext.fwd(*args, True, "mamba")
+    dout = torch.randn(out.shape, generator=g).cuda()
+    want = ext.bwd(*args, dout, x.clone(), out, None, True, False, "mamba")
+    room = torch.full((24 * 2500,), float("nan"), device="cuda")       # more than any spacing needs; on both sides of the states
+    call = _lib.call
+
+    def patched(fn, a, stream):
+        if fn == "b200_selscan_bwd":
+            f = a.f
+            f.stage_h, f.stage_len = room.data_ptr() + 4 * 16 * 1024, stage_len
+            a.f = f
+        else:
+            a.stage_h, a.stage_len = room.data_ptr() + 4 * 16 * 1024, stage_len
+        call(fn, a, stream)
+
+    monkeypatch.setattr(_lib, "call", patched)
+    again, x, _ = ext.fwd(*args, True, "mamba")
+    assert torch.equal(again, out) and bool(room.isnan().all())
+    got = ext.bwd(*args, dout, x.clone(), out, None, True, False, "mamba")
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert_close(a.cpu(), b.cpu(), rtol=2e-5, atol_scale=2e-6, name=f"gradient {i}")

@@ -61,6 +61,26 @@ def test_null_and_range_checks_return_errors_without_launching():
     assert lib.b200_ssu_step(ctypes.byref(u), None) == _lib.enum("B200_ERR_NULL")
 
 
+def test_selscan_bwd_refuses_a_misaligned_workspace():
+    """Its boundary states are written 32 bytes at a time."""
+    lib = _lib.lib()
+    buf = (ctypes.c_float * 4096)()
+    p = -(-ctypes.addressof(buf) // 32) * 32
+    q = _lib.struct("b200_selscan_bwd_args")()
+    f = _lib.struct("b200_selscan_fwd_args")()
+    f.batch = f.dim = f.n_groups = f.var_B = f.var_C = 1
+    f.seqlen, f.dstate, f.method = 8, 16, _lib.enum("B200_DISC_MAMBA")
+    f.u = f.delta = f.A = f.B = f.C = f.out = f.x = p
+    f.A_ns, f.B_ns, f.C_ns = 1, 8, 8
+    q.f = f
+    q.dout = q.du = q.ddelta = q.dA = q.dB = q.dC = p
+    q.work_bytes = lib.b200_selscan_bwd_work_bytes(ctypes.byref(q))
+    assert q.work_bytes > 0
+    q.work = p + 16
+    assert lib.b200_selscan_bwd(ctypes.byref(q), None) == _lib.enum("B200_ERR_ALIGN")
+    assert b"32-byte" in lib.b200_last_error()
+
+
 def test_scratch_size_query():
     lib = _lib.lib()
     assert lib.b200_s4_bwd_scratch_bytes(0, 1, 1) == 0

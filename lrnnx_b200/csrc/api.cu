@@ -114,7 +114,8 @@ int b200_selscan_bwd(const b200_selscan_bwd_args *args, void *stream) {
   if (!args->h_in && !args->q_in && selscan_row1_supported(f)) return selscan_row1_bwd(*args, st);
   if (!selscan_seq_bwd_supported(*args)) return selscan_bwd_generic(*args, st);
   b200_selscan_bwd_args a = *args;
-  if (!stage_usable(a.f.stage_len)) a.f.stage_h = nullptr;
+  // the forward's stage states start from zero: with a state entering the sequence they are not its states
+  if (!stage_usable(a.f.stage_len) || a.h_in) a.f.stage_h = nullptr;
   B200_REQUIRE((reinterpret_cast<uintptr_t>(a.work) & 31) == 0, B200_ERR_ALIGN, "selscan_bwd: work must be 32-byte aligned");
   if (a.work) return selscan_seq_bwd(a, a.work, a.work_bytes, st);
   void *work = nullptr;

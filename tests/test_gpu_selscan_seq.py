@@ -121,3 +121,31 @@ def test_stage_states_of_another_spacing(stage_len, monkeypatch):
     got = ext.bwd(*args, dout, x.clone(), out, None, True, False, "mamba")
     for i, (a, b) in enumerate(zip(got, want)):
         assert_close(a.cpu(), b.cpu(), rtol=2e-5, atol_scale=2e-6, name=f"gradient {i}")
+
+
+def test_entering_state_beside_stage_states(monkeypatch):
+    """h_in together with the stage states of the zero-start forward, as a caller of the C entry points may hand them
+    over: the gradients are those of the entering state."""
+    from lrnnx_b200 import _lib
+    from lrnnx_b200 import selective_scan_cuda as ext
+    t, g = _make_inputs(2, 24, 16, 700, seed=2, with_z=False)
+    c = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in t.items()}
+    args = (c["u"], c["delta"], c["A"], c["B"], c["C"], c["D"], None, c["delta_bias"], None)
+    out, x = ext.fwd(*args, True, "mamba")
+    h_in = torch.randn(2, 24, 16, generator=g).cuda()
+    dout = torch.randn(out.shape, generator=g).cuda()
+    want = ext.bwd(*args, dout, x, out, None, True, False, "mamba", h_in=h_in)
+    ptr, stage_len = ext._stage_states_of(x, 2, 24, 700, 16)
+    assert stage_len > 0
+    call = _lib.call
+
+    def patched(fn, a, stream):
+        f = a.f
+        f.stage_h, f.stage_len = ptr, stage_len
+        a.f = f
+        call(fn, a, stream)
+
+    monkeypatch.setattr(_lib, "call", patched)
+    got = ext.bwd(*args, dout, x, out, None, True, False, "mamba", h_in=h_in)
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert_close(a.cpu(), b.cpu(), rtol=2e-5, atol_scale=2e-6, name=f"gradient {i}")

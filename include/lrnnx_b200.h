@@ -151,9 +151,10 @@ typedef struct b200_selscan_bwd_args {
    * sequence send back (b200_selscan_adjoint_summary, folded from the right). */
   const void *h_in, *q_in;
   /* Device workspace of the state-parallel kernels, 32-byte aligned, free again when the call's work
-   * on `stream` is done: b200_selscan_bwd_work_bytes() bytes are enough (with fewer the batch is
-   * processed in thinner slices).  NULL: the call takes it from the stream-ordered allocator
-   * (cudaMallocAsync) and returns it on the same stream. */
+   * on `stream` is done: b200_selscan_bwd_work_bytes() bytes, at most 2 GiB, are enough.  With fewer the
+   * call runs in thinner slices of the batch, of the sequence and at last of the channels; 64 KiB + 64 bytes
+   * (one channel and 2048 steps) are the least.  NULL: the call takes it from the stream-ordered allocator
+   * (cudaMallocAsync) and returns it on the same stream; without memory it runs on kernels that need none. */
   void *work;
   int64_t work_bytes;
 } b200_selscan_bwd_args;

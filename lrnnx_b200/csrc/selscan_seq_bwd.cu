@@ -75,6 +75,8 @@ template <typename T> struct Quad<T, true> {
 // what the launch needs beyond the call's arguments
 struct SeqPre {
   float4 *hs, *qs;       // (batch, dim, 4 quarters of the states, seq_blocks(seqlen))
+  float4 *carry;         // (batch, dim, 4): the adjoint that leaves the window to the left
+  int t0, total;         // the call's arguments are steps t0 .. t0 + seqlen of this many; x and stage_h those of all
   int piece;             // steps per independently started piece of the states' walk
   int tiles;             // thread blocks that a batch row takes
   int adj;               // thread blocks of the first kind: one per tile and batch row, then one per piece
@@ -170,15 +172,18 @@ __device__ __forceinline__ void seq_walk(const b200_selscan_bwd_args &a, const S
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);                    // the state, or q
   if (mine) {
     const int64_t o = QS * q;
-    const int n_chunks = (p.seqlen + kChunk - 1) / kChunk;
-    const float *first = reinterpret_cast<const float *>(ADJ ? a.q_in : a.h_in);
-    if (t_begin == 0) {
-      if (first) v = *reinterpret_cast<const float4 *>(first + row * QN + o);
+    const int t = x.t0 + t_begin;                                // a multiple of the piece
+    if (ADJ) {
+      if (x.t0 + p.seqlen < x.total) v = x.carry[row * 4 + q];
+      else if (a.q_in) v = *reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(a.q_in) + row * QN + o);
+    } else if (t == 0) {
+      if (a.h_in) v = *reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(a.h_in) + row * QN + o);
     } else if (p.stage_h) {
-      const int64_t n_stages = (p.seqlen + p.stage_len - 1) / p.stage_len;
-      v = *reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p.stage_h) + (row * n_stages + t_begin / p.stage_len - 1) * QN + o);
+      const int64_t n_stages = (x.total + p.stage_len - 1) / p.stage_len;
+      v = *reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p.stage_h) + (row * n_stages + t / p.stage_len - 1) * QN + o);
     } else {
-      const float4 *xr = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p.x) + (row * n_chunks + t_begin / kChunk - 1) * 2 * QN + 2 * o);
+      const int64_t n_chunks = (x.total + kChunk - 1) / kChunk;
+      const float4 *xr = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p.x) + (row * n_chunks + t / kChunk - 1) * 2 * QN + 2 * o);
       v = make_float4(xr[0].y, xr[0].w, xr[1].y, xr[1].w);
     }
   }
@@ -277,6 +282,7 @@ __device__ __forceinline__ void seq_walk(const b200_selscan_bwd_args &a, const S
     out += dir / kSeqBlock;
     __syncwarp();
   }
+  if (ADJ && mine && x.t0 > 0) x.carry[row * 4 + q] = make_float4(s0.x, s0.y, s1.x, s1.y);
 }
 
 template <typename T, bool ALN, bool Z>
@@ -596,14 +602,21 @@ template <typename T> bool quads_aligned(const b200_selscan_bwd_args &a) {
          ok(p.out_z, p.out_z_bs, p.out_z_ds) && ok(a.du, a.du_bs, a.du_ds) && ok(a.ddelta, a.ddelta_bs, a.ddelta_ds);
 }
 
-template <typename T> int launch_bwd(const b200_selscan_bwd_args &a, float4 *hs, float4 *qs, cudaStream_t st) {
+// a: a window of `total` steps that begins at step t0, as a call of its own (x and stage_h aside)
+template <typename T> int launch_bwd(const b200_selscan_bwd_args &a, int t0, int total, void *work, cudaStream_t st) {
   const b200_selscan_fwd_args &f = a.f;
   const int cpg = f.dim / f.n_groups;
+  // the carry comes first: it lies in the same place for windows of any length
+  const int64_t rows4 = (int64_t)f.batch * f.dim * 4;
+  float4 *carry = reinterpret_cast<float4 *>(work), *hs = carry + rows4, *qs = hs + rows4 * seq_blocks(f.seqlen);
   // 1. states and adjoints.  Pieces of the states' walk start where the forward call left a state: every
   // 256 steps is enough parallelism; without stage states only the 2048-step checkpoints of x are there
   SeqPre x{};
   x.hs = hs;
   x.qs = qs;
+  x.carry = carry;
+  x.t0 = t0;
+  x.total = total;
   x.piece = f.stage_h ? kStage : kChunk;
   x.tiles = f.n_groups * ((cpg + FW * QCH - 1) / (FW * QCH));
   x.adj = f.batch * x.tiles;
@@ -641,18 +654,88 @@ template <typename T> int launch_bwd(const b200_selscan_bwd_args &a, float4 *hs,
   return launch_status();
 }
 
-int64_t row_bytes(const b200_selscan_fwd_args &f) {       // hs and qs of one batch row
-  return 2 * (int64_t)seq_blocks(f.seqlen) * f.dim * QN * (int64_t)sizeof(float);
+// the workspace of one channel of one batch row over `steps` steps: carry, hs, qs
+int64_t channel_bytes(int steps) { return 2 * (int64_t)seq_blocks(steps) * QN * 4 + QN * 4; }
+
+// One launch's share of the call: batch rows, channels (whole groups, or part of one) and steps from these on.
+struct Slice {
+  int b0, rows, c0, chans, t0, steps;
+};
+// How many channels of a row a workspace of `room` channels takes at a time: whole groups; or less than one group, then
+// whole thread blocks or whole warps of the walks where there is room for one.
+int slice_channels(const b200_selscan_fwd_args &f, int64_t room) {
+  const int cpg = f.dim / f.n_groups;
+  if (room >= cpg) return (int)(room / cpg < f.n_groups ? room / cpg : f.n_groups) * cpg;
+  const int n = (int)room;
+  return n >= FW * QCH ? n / (FW * QCH) * (FW * QCH) : n >= QCH ? n / QCH * QCH : n;
+}
+
+int run_slice(const b200_selscan_bwd_args &a, const Slice &w, void *work, cudaStream_t st) {
+  const int es = act_size(a.f.dtype), total = a.f.seqlen;
+  const int cpg = a.f.dim / a.f.n_groups, g0 = w.c0 / cpg;
+  b200_selscan_bwd_args s = a;
+  b200_selscan_fwd_args &f = s.f;
+  f.batch = w.rows;
+  f.dim = w.chans;
+  f.seqlen = w.steps;
+  f.n_groups = w.chans > cpg ? w.chans / cpg : 1;
+  const int64_t n_chunks = (total + kChunk - 1) / kChunk, row0 = (int64_t)w.b0 * a.f.dim + w.c0;
+  const auto at = [](const void *p, int64_t bytes) { return p ? (void *)(const_cast<char *>(reinterpret_cast<const char *>(p)) + bytes) : nullptr; };
+  const auto act = [&](const void *p, int64_t bs, int64_t ds) { return at(p, (w.b0 * bs + w.c0 * ds + w.t0) * es); };
+  f.u = act(f.u, f.u_bs, f.u_ds);
+  f.delta = act(f.delta, f.delta_bs, f.delta_ds);
+  f.z = act(f.z, f.z_bs, f.z_ds);
+  f.out = act(f.out, f.out_bs, f.out_ds);
+  f.out_z = act(f.out_z, f.out_z_bs, f.out_z_ds);
+  f.B = at(f.B, (w.b0 * f.B_bs + g0 * f.B_gs + w.t0) * es);
+  f.C = at(f.C, (w.b0 * f.C_bs + g0 * f.C_gs + w.t0) * es);
+  f.A = at(f.A, w.c0 * f.A_ds * 4);
+  f.D = at(f.D, (int64_t)w.c0 * 4);
+  f.delta_bias = at(f.delta_bias, (int64_t)w.c0 * 4);
+  f.x = at(f.x, row0 * n_chunks * 2 * QN * 4);
+  if (f.stage_h) f.stage_h = at(f.stage_h, row0 * ((total + f.stage_len - 1) / f.stage_len) * QN * 4);
+  s.dout = act(s.dout, s.dout_bs, s.dout_ds);
+  s.du = act(s.du, s.du_bs, s.du_ds);
+  s.ddelta = act(s.ddelta, s.ddelta_bs, s.ddelta_ds);
+  s.dz = act(s.dz, s.dz_bs, s.dz_ds);
+  s.dA = at(s.dA, w.c0 * s.dA_ds * 4);
+  s.dB = at(s.dB, (w.b0 * s.dB_bs + g0 * s.dB_gs + w.t0) * 4);
+  s.dC = at(s.dC, (w.b0 * s.dC_bs + g0 * s.dC_gs + w.t0) * 4);
+  s.dD = at(s.dD, (int64_t)w.c0 * 4);
+  s.ddelta_bias = at(s.ddelta_bias, (int64_t)w.c0 * 4);
+  s.h_in = at(s.h_in, row0 * QN * 4);
+  s.q_in = at(s.q_in, row0 * QN * 4);
+  if (f.dtype == B200_F32) return launch_bwd<float>(s, w.t0, total, work, st);
+  if (f.dtype == B200_BF16) return launch_bwd<__nv_bfloat16>(s, w.t0, total, work, st);
+  return launch_bwd<__half>(s, w.t0, total, work, st);
+}
+
+// How a call is cut for a workspace of so many bytes: into batch rows while one fits; one row into windows of the
+// sequence, from the last to the first, which keeps all its channels in flight (the adjoint is one serial walk however
+// it is cut); and only where not even the shortest window of all channels fits into channels as well.
+struct Cut {
+  int rows, chans, steps;        // rows < 1: not even one channel fits
+};
+Cut cut_of(const b200_selscan_fwd_args &f, int64_t bytes) {
+  const int64_t row = channel_bytes(f.seqlen) * f.dim;
+  if (bytes >= row) return {(int)(bytes / row < f.batch ? bytes / row : f.batch), f.dim, f.seqlen};
+  const int window = f.seqlen < kChunk ? f.seqlen : kChunk;      // windows begin where a checkpoint is
+  if (bytes >= channel_bytes(window) * f.dim) {
+    int64_t n = bytes / (channel_bytes(window) * f.dim);
+    while (channel_bytes((int)(n + 1) * window) * f.dim <= bytes) ++n;      // one carry for all of them
+    return {1, f.dim, (int)n * window};
+  }
+  const int64_t room = bytes / channel_bytes(window);
+  return {room < 1 ? 0 : 1, room < 1 ? 0 : slice_channels(f, room), window};
 }
 
 }  // namespace
 
-// Transient device memory of the backward call: the states and adjoints of a slice of the batch.
-// A slice holds at most 2 GiB of them (a single batch row may need more).
+// Transient device memory of the backward call: the states and adjoints of a slice, 32 bytes per channel and step.
+// A slice holds at most 2 GiB of them.
 int64_t selscan_seq_bwd_bytes(const b200_selscan_fwd_args &f) {
-  const int64_t row = row_bytes(f), most = (int64_t)2 << 30;
-  const int64_t rows = most / row < 1 ? 1 : most / row;
-  return row * (rows < f.batch ? rows : f.batch);
+  const Cut c = cut_of(f, (int64_t)2 << 30);
+  return channel_bytes(c.steps) * c.chans * c.rows;
 }
 
 bool selscan_seq_bwd_supported(const b200_selscan_bwd_args &a) {
@@ -667,41 +750,17 @@ bool selscan_seq_bwd_supported(const b200_selscan_bwd_args &a) {
 }
 
 int selscan_seq_bwd(const b200_selscan_bwd_args &a, void *work, int64_t work_bytes, cudaStream_t st) {
-  const int64_t row = row_bytes(a.f);
-  const int es = act_size(a.f.dtype);
-  const int rows = (int)(work_bytes / row < a.f.batch ? work_bytes / row : a.f.batch);
-  B200_REQUIRE(rows >= 1, B200_ERR_SHAPE, "selscan_bwd: the workspace is too small for one batch row");
-  float4 *hs = reinterpret_cast<float4 *>(work);
-  float4 *qs = hs + (int64_t)rows * (row / 2 / (int64_t)sizeof(float4));
-  const auto at = [](const void *p, int64_t bytes) { return p ? (void *)(const_cast<char *>(reinterpret_cast<const char *>(p)) + bytes) : nullptr; };
-  for (int b0 = 0; b0 < a.f.batch; b0 += rows) {
-    b200_selscan_bwd_args s = a;
-    b200_selscan_fwd_args &f = s.f;
-    f.batch = rows < a.f.batch - b0 ? rows : a.f.batch - b0;
-    f.u = at(f.u, b0 * f.u_bs * es);
-    f.delta = at(f.delta, b0 * f.delta_bs * es);
-    f.z = at(f.z, b0 * f.z_bs * es);
-    f.out = at(f.out, b0 * f.out_bs * es);
-    f.out_z = at(f.out_z, b0 * f.out_z_bs * es);
-    f.B = at(f.B, b0 * f.B_bs * es);
-    f.C = at(f.C, b0 * f.C_bs * es);
-    const int64_t n_chunks = (f.seqlen + kChunk - 1) / kChunk;
-    f.x = at(f.x, b0 * (int64_t)f.dim * n_chunks * 2 * QN * 4);
-    if (f.stage_h) f.stage_h = at(f.stage_h, b0 * (int64_t)f.dim * ((f.seqlen + f.stage_len - 1) / f.stage_len) * QN * 4);
-    s.dout = at(s.dout, b0 * s.dout_bs * es);
-    s.du = at(s.du, b0 * s.du_bs * es);
-    s.ddelta = at(s.ddelta, b0 * s.ddelta_bs * es);
-    s.dz = at(s.dz, b0 * s.dz_bs * es);
-    s.dB = at(s.dB, b0 * s.dB_bs * 4);
-    s.dC = at(s.dC, b0 * s.dC_bs * 4);
-    s.h_in = at(s.h_in, b0 * (int64_t)f.dim * QN * 4);
-    s.q_in = at(s.q_in, b0 * (int64_t)f.dim * QN * 4);
-    int e;
-    if (f.dtype == B200_F32) e = launch_bwd<float>(s, hs, qs, st);
-    else if (f.dtype == B200_BF16) e = launch_bwd<__nv_bfloat16>(s, hs, qs, st);
-    else e = launch_bwd<__half>(s, hs, qs, st);
-    if (e) return e;
-  }
+  const int dim = a.f.dim, cpg = dim / a.f.n_groups, L = a.f.seqlen;
+  const Cut cut = cut_of(a.f, work_bytes);
+  B200_REQUIRE(cut.rows >= 1, B200_ERR_SHAPE, "selscan_bwd: the workspace is too small for one channel and %d steps", cut.steps);
+  for (int b = 0; b < a.f.batch; b += cut.rows)
+    for (int c = 0, n; c < dim; c += n) {
+      n = cut.chans < dim - c ? cut.chans : dim - c;
+      if (cut.chans < cpg && n > cpg - c % cpg) n = cpg - c % cpg;      // not past the end of a group
+      const int rows = cut.rows < a.f.batch - b ? cut.rows : a.f.batch - b;
+      for (int t = (L - 1) / cut.steps * cut.steps; t >= 0; t -= cut.steps)
+        if (int e = run_slice(a, {b, rows, c, n, t, cut.steps < L - t ? cut.steps : L - t}, work, st)) return e;
+    }
   return 0;
 }
 

@@ -289,6 +289,17 @@ def fwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, delta_softplus, discret
     return [out, x] if out_z is None else [out, x, out_z]
 
 
+def _workspace(numel, device):
+    """A workspace of up to ``numel`` bytes: a quarter of it, and so on, where there is no memory for it (the call then
+    runs in thinner slices), and None where not even a megabyte is left (the kernels that need none take the call)."""
+    while numel > 0:
+        try:
+            return torch.empty(numel, dtype=torch.uint8, device=device)
+        except torch.cuda.OutOfMemoryError:
+            numel = numel // 4 if numel >= 1 << 22 else 0
+    return None
+
+
 def bwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, dout, x_, out_, dz_, delta_softplus, recompute_out_z,
         discretization_method_str, h_in=None, q_in=None):
     """Returns ``[du, ddelta, dA, dB, dC, dD, ddelta_bias, (ddeltaA), (dz), (out_z)]``
@@ -387,10 +398,9 @@ def bwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, dout, x_, out_, dz_, de
         else:
             q.dC_bs, q.dC_gs, q.dC_ns = 0, dC.stride(0), dC.stride(1)
         q.f = f
-        work_bytes = _lib.lib().b200_selscan_bwd_work_bytes(ctypes.byref(q))
-        if work_bytes > 0:
-            work = torch.empty(work_bytes, dtype=torch.uint8, device=u.device)
-            q.work, q.work_bytes = work.data_ptr(), work_bytes
+        work = _workspace(_lib.lib().b200_selscan_bwd_work_bytes(ctypes.byref(q)), u.device)
+        if work is not None:
+            q.work, q.work_bytes = work.data_ptr(), work.numel()
         _lib.call("b200_selscan_bwd", q, _stream(u))
         result = [du, ddelta, dA, dB.to(B.dtype), dC.to(C.dtype), dD, ddelta_bias]
         if deltaA_ is not None:

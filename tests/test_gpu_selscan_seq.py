@@ -149,3 +149,42 @@ def test_entering_state_beside_stage_states(monkeypatch):
     got = ext.bwd(*args, dout, x, out, None, True, False, "mamba", h_in=h_in)
     for i, (a, b) in enumerate(zip(got, want)):
         assert_close(a.cpu(), b.cpu(), rtol=2e-5, atol_scale=2e-6, name=f"gradient {i}")
+
+
+@pytest.mark.parametrize("dim,groups", [(24, 1), (36, 3), (80, 1)])
+@pytest.mark.parametrize("states", ["saved", "checkpoints", "entering"])
+def test_slices_of_the_backward(dim, groups, states, monkeypatch):
+    """Workspaces that hold a window of the sequence (two and one checkpoint chunks), whole groups, part of a group and a
+    single channel, of a length that leaves the last window ragged; with the forward's stage states, with its checkpoints
+    alone, and with a state and an adjoint that enter the sequence."""
+    from lrnnx_b200 import _lib
+    from lrnnx_b200 import selective_scan_cuda as ext
+    batch, L = 2, 3 * 2048 + 37
+    t, g = _make_inputs(batch, dim, 16, L, seed=dim, groups=groups)
+    c = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in t.items()}
+    args = (c["u"], c["delta"], c["A"], c["B"], c["C"], c["D"], c["z"], c["delta_bias"], None)
+    out, x, _ = ext.fwd(*args, True, "mamba")
+    dout = torch.randn(out.shape, generator=g).cuda()
+    kw = {k: torch.randn(batch, dim, 16, generator=g).cuda() for k in ("h_in", "q_in")} if states == "entering" else {}
+    if states == "checkpoints":
+        x = x.clone()
+    call, sizes = _lib.call, []
+
+    def patched(fn, a, stream):
+        if fn == "b200_selscan_bwd":
+            sizes.append(a.work_bytes)
+            a.work_bytes = sizes[-1] if size is None else size
+        call(fn, a, stream)
+
+    monkeypatch.setattr(_lib, "call", patched)
+    channel = 2048 * 32 + 64
+    size = None
+    want = ext.bwd(*args, dout, x, out, None, True, False, "mamba", **kw)
+    for size in (2 * channel * dim, channel * dim, channel * (dim // groups), channel * 9, channel):
+        assert size < sizes[0]
+        got = ext.bwd(*args, dout, x, out, None, True, False, "mamba", **kw)
+        for i, (a, b) in enumerate(zip(got, want)):
+            assert_close(a.cpu(), b.cpu(), rtol=2e-5, atol_scale=2e-6, name=f"{size // channel} channels, gradient {i}")
+    size = channel - 1
+    with pytest.raises(RuntimeError, match="too small"):
+        ext.bwd(*args, dout, x, out, None, True, False, "mamba", **kw)

@@ -81,6 +81,37 @@ def test_selscan_bwd_refuses_a_misaligned_workspace():
     assert b"32-byte" in lib.b200_last_error()
 
 
+@pytest.mark.parametrize("batch,dim,seqlen,groups", [(8, 1536, 2048, 1), (1, 5120, 131072, 1), (1, 2560, 1 << 20, 1), (2, (1 << 18) + 32, 4096, 1),
+                                                     (1, 1 << 20, 100, 1 << 10), (1, 8, 1 << 28, 8)])
+def test_selscan_bwd_workspace_is_bounded(batch, dim, seqlen, groups):
+    lib = _lib.lib()
+    q = _lib.struct("b200_selscan_bwd_args")()
+    f = _lib.struct("b200_selscan_fwd_args")()
+    f.batch, f.dim, f.n_groups, f.seqlen, f.dstate = batch, dim, groups, seqlen, 16
+    f.method, f.var_B, f.var_C = _lib.enum("B200_DISC_MAMBA"), 1, 1
+    f.u = f.delta = f.A = f.B = f.C = f.x = 1 << 20
+    q.f = f
+    assert 0 < lib.b200_selscan_bwd_work_bytes(ctypes.byref(q)) <= 2 << 30
+
+
+def test_selscan_bwd_workspace_shrinks_without_memory(monkeypatch):
+    """The call takes what the allocator has, and goes without where it has nothing."""
+    from lrnnx_b200 import selective_scan_cuda as ext
+    empty, room = torch.empty, [0]
+
+    def limited(n, **kw):
+        if n > room[0]:
+            raise torch.cuda.OutOfMemoryError
+        return empty(n, dtype=torch.uint8)
+
+    monkeypatch.setattr(torch, "empty", limited)
+    for have, got in ((1 << 40, 3 << 28), (1 << 29, 3 << 26), (1 << 22, 3 << 20), (1 << 10, None)):
+        room[0] = have
+        work = ext._workspace(3 << 28, "cuda")
+        assert (None if work is None else work.numel()) == got
+    assert ext._workspace(0, "cuda") is None
+
+
 def test_scratch_size_query():
     lib = _lib.lib()
     assert lib.b200_s4_bwd_scratch_bytes(0, 1, 1) == 0

@@ -448,8 +448,8 @@ selscan_seq_bwd_kernel(const b200_selscan_bwd_args a, const float4 *__restrict__
 #pragma unroll
     for (int k = 0; k < BW; ++k) {
       const int n = left > 0 && i + k < i_end ? 16 : 0;
-      cp16(&sm.st[buf][k][0][warp][lane], hp, n);
-      cp16(&sm.st[buf][k][1][warp][lane], qp, n);
+      cp16(&sm.st[buf][k][0][warp][lane], n ? hp : hs, n);          // copies of 0 bytes name a mapped address too
+      cp16(&sm.st[buf][k][1][warp][lane], n ? qp : qs, n);
       hp += sd;
       qp += sd;
     }

@@ -46,7 +46,7 @@ def selective_state_update(state, x, dt, A, B, C, D=None, z=None, dt_bias=None, 
     """state (batch, dim, dstate) or (batch, nheads, dim, dstate), updated in place;
     x, dt, z, deltaA (batch, dim) or (batch, nheads, dim); A (dim, dstate) or (nheads, dim, dstate);
     B, C (batch, dstate) or (batch, ngroups, dstate); D, dt_bias (dim,) or (nheads, dim).
-    Returns out with the shape and dtype of x."""
+    Returns out with the dtype of x: (batch, nheads, dim) for a state with heads, (batch, dim) otherwise."""
     has_heads = state.dim() > 3
     (_, nheads, dim, dstate), s_state = _heads(state, 4)
     x_shape, s_x = _heads(x, 3)
@@ -117,4 +117,6 @@ def selective_state_update(state, x, dt, A, B, C, D=None, z=None, dt_bias=None, 
         if state_batch_indices is not None:
             a.state_batch_indices = state_batch_indices.data_ptr()
         _lib.call("b200_ssu_step", a, _lib.stream_of(x))
-    return out if has_heads or out.dim() == 2 else out.squeeze(1)
+    if has_heads:
+        return out if out.dim() == 3 else out.unsqueeze(1)
+    return out if out.dim() == 2 else out.squeeze(1)

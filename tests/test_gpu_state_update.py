@@ -221,3 +221,20 @@ def test_s7_with_deltaA_is_refused():
     with pytest.raises(RuntimeError, match="deltaA is not defined for the s7"):
         selective_state_update(state, **args, deltaA=torch.rand_like(args["x"]), discretization="s7")
     assert torch.equal(state, before)
+
+
+@pytest.mark.parametrize("state_heads", [False, True])
+@pytest.mark.parametrize("x_heads", [False, True])
+def test_shape_of_the_result(state_heads, x_heads):
+    """The result has a heads dimension where the state has one, whatever x has."""
+    from lrnnx_b200.ops import selective_state_update
+    g = torch.Generator().manual_seed(3)
+    r = lambda *s: torch.randn(*s, generator=g).cuda()
+    batch, dim, N = 3, 20, 16
+    state, x, dt, A, B, C = r(batch, dim, N), r(batch, dim), r(batch, dim), -r(dim, N).abs(), r(batch, N), r(batch, N)
+    want = selective_state_update(state.clone(), x, dt, A, B, C, dt_softplus=True)
+    assert want.shape == (batch, dim)
+    got = selective_state_update(state.clone().unsqueeze(1) if state_heads else state.clone(), x.unsqueeze(1) if x_heads else x, dt, A, B, C,
+                                 dt_softplus=True)
+    assert got.shape == ((batch, 1, dim) if state_heads else (batch, dim))
+    assert torch.equal(got.reshape(batch, dim), want)

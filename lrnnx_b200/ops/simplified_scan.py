@@ -59,7 +59,8 @@ class SimplifiedScanFn(torch.autograd.Function):
         dstate = A_k.shape[1]
         Bu = _proj(B, u, padded=True)
         ident = torch.ones(P, dstate, dtype=A.dtype, device=A.device)
-        out, xs = simplified_scan_cuda.fwd(Bu, delta, A_k, ident, ident, deltaA, discretization)
+        out, xs = simplified_scan_cuda.fwd(Bu, delta, A_k, ident, ident, deltaA, discretization,
+                                           padded=projection.fits(C, Bu))
         y = _proj(C, out)
         ctx.discretization = discretization
         ctx.has_deltaA = deltaA is not None
@@ -79,7 +80,8 @@ class SimplifiedScanFn(torch.autograd.Function):
         if dx_out.stride(-1) != 1:
             dx_out = dx_out.contiguous()
         res = simplified_scan_cuda.bwd(Bu, delta, A_k, ident, ident, deltaA, dx_out, xs, ctx.discretization,
-                                      need_dB_dC=False, out_=out if out.stride(-1) == 1 else None)
+                                      need_dB_dC=False, out_=out if out.stride(-1) == 1 else None,
+                                      padded=projection.fits(B.t(), Bu))
         dBu, ddelta, dA = res[0], res[1], res[2]
         ddeltaA = res[5] if ctx.has_deltaA else None
         du = _proj(B, dBu, conj_transpose=True)
@@ -111,7 +113,8 @@ class S5InnerFn(torch.autograd.Function):
         dstate = A_k.shape[1]
         Bu = _proj(B, u, padded=True)
         ident = torch.ones(P, dstate, dtype=A.dtype, device=A.device)
-        scan_out, xs = simplified_scan_cuda.fwd(Bu, delta, A_k, ident, ident, deltaA, discretization)
+        scan_out, xs = simplified_scan_cuda.fwd(Bu, delta, A_k, ident, ident, deltaA, discretization,
+                                                padded=projection.fits(C, Bu))
         y_complex = _proj(C, scan_out)
         y_real = 2 * y_complex.real if conj_sym else y_complex.real
         u_real = u.real if u.is_complex() else u
@@ -136,7 +139,8 @@ class S5InnerFn(torch.autograd.Function):
         if dscan.stride(-1) != 1:
             dscan = dscan.contiguous()
         res = simplified_scan_cuda.bwd(Bu, delta, A_k, ident, ident, deltaA, dscan, xs, ctx.discretization,
-                                      need_dB_dC=False, out_=scan_out if scan_out.stride(-1) == 1 else None)
+                                      need_dB_dC=False, out_=scan_out if scan_out.stride(-1) == 1 else None,
+                                      padded=projection.fits(B.t(), Bu))
         dBu, ddelta, dA = res[0], res[1], res[2]
         ddeltaA = res[5] if ctx.has_deltaA else None
         du_scan = _proj(B, dBu, conj_transpose=True)

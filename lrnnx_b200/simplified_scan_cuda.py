@@ -60,20 +60,21 @@ def _stream(t) -> int:
     return _lib.stream_of(t)
 
 
-def _like(u):
-    """An output for u: with u's rows where they are padded to an even pitch, dense otherwise."""
-    L = u.shape[2]
-    if u.stride() == (u.shape[1] * (L + 1), L + 1, 1):
-        return torch.empty_strided(u.shape, u.stride(), dtype=u.dtype, device=u.device)
-    return torch.empty_like(u)
+def _rows(u, padded):
+    """An output for u: like u, or in rows of an even pitch, which the projection kernels read in place."""
+    if not padded:
+        return torch.empty_like(u)
+    batch, dim, L = u.shape
+    return torch.empty((batch, dim, L + L % 2), dtype=u.dtype, device=u.device)[..., :L]
 
 
-def fwd(u, delta, A, B, C, deltaA_, discretization_method_str):
-    """Returns ``[out, x]``: out complex64 like u, x (batch, dim, n_chunks, 2*dstate) complex64."""
+def fwd(u, delta, A, B, C, deltaA_, discretization_method_str, padded=False):
+    """Returns ``[out, x]``: out complex64 like u, x (batch, dim, n_chunks, 2*dstate) complex64.  An addition to the
+    reference signature: ``padded=True`` lays out's rows out with an even pitch."""
     a, (batch, dim, seqlen, dstate) = _common(u, delta, A, B, C, deltaA_, discretization_method_str)
     n_chunks = (seqlen + CHUNK - 1) // CHUNK
     with _lib.on_device(u):
-        out = _like(u)
+        out = _rows(u, padded)
         x = torch.empty((batch, dim, n_chunks, 2 * dstate), dtype=torch.complex64, device=u.device)
         a.out, a.x = out.data_ptr(), x.data_ptr()
         a.out_bs, a.out_ds = out.stride(0), out.stride(1)
@@ -81,12 +82,14 @@ def fwd(u, delta, A, B, C, deltaA_, discretization_method_str):
     return [out, x]
 
 
-def bwd(u, delta, A, B, C, deltaA_, dout, x_, discretization_method_str, need_dB_dC=True, out_=None):
+def bwd(u, delta, A, B, C, deltaA_, dout, x_, discretization_method_str, need_dB_dC=True, out_=None,
+        padded=False):
     """Returns ``[du, ddelta, dA, dB, dC]`` plus ``ddeltaA`` when deltaA was given
-    (simplified_scan_cpu.cpp:328-330).  Two additions to the reference signature, for single-state
-    rows: ``need_dB_dC=False`` skips the dB / dC sums and returns None in their place; ``out_``, the
-    output of ``fwd`` for the same arguments, lets the kernel take the states from it instead of
-    recomputing them (B C must be non-zero)."""
+    (simplified_scan_cpu.cpp:328-330).  Additions to the reference signature: ``padded=True`` lays
+    du's rows out with an even pitch; for single-state rows, ``need_dB_dC=False`` skips the dB / dC
+    sums and returns None in their place, and ``out_``, the output of ``fwd`` for the same
+    arguments, lets the kernel take the states from it instead of recomputing them (B C must be
+    non-zero)."""
     a, (batch, dim, seqlen, dstate) = _common(u, delta, A, B, C, deltaA_, discretization_method_str)
     _check(dout.dtype == torch.complex64 and dout.is_cuda, "dout must be a complex64 CUDA tensor")
     _check(dout.stride(-1) == 1 or dout.size(-1) == 1, "dout must be contiguous in the last dimension")
@@ -99,7 +102,7 @@ def bwd(u, delta, A, B, C, deltaA_, dout, x_, discretization_method_str, need_dB
                "x must be a contiguous complex64 CUDA tensor")
         _check(tuple(x_.shape) == (batch, dim, n_chunks, 2 * dstate), "x has the wrong shape")
     with _lib.on_device(u):
-        du = _like(u)
+        du = _rows(u, padded)
         ddelta = torch.empty_like(delta)
         if A.is_contiguous() and B.is_contiguous() and C.is_contiguous():
             dA, dB, dC = torch.zeros((3,) + tuple(A.shape), dtype=A.dtype, device=A.device).unbind(0)  # one fill

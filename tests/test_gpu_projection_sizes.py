@@ -68,3 +68,17 @@ def test_simplified_scan_at_odd_lengths(L):
     want = run(O.simplified_scan_oracle, wide, compute_dtype=torch.float64)
     for a, b in zip(run(simplified_scan_fn, lambda v: v.cuda()), want):
         assert float((wide(a) - b).abs().max()) <= 1e-5 * float(b.abs().max())
+
+
+@pytest.mark.parametrize("L", [63, 64])
+def test_the_extension_lays_its_outputs_out_as_before(L):
+    """A caller's own view of rows that are one element longer gets dense outputs, as any other input; padded rows are for
+    callers that ask for them."""
+    from lrnnx_b200 import simplified_scan_cuda as ext
+    g = torch.Generator().manual_seed(L)
+    u, dout = _cn(g, 2, 40, L + 1)[..., :L], _cn(g, 2, 40, L + 1)[..., :L]
+    delta, A, one = torch.ones(2, 40, L, device="cuda"), -torch.rand(40, 1, device="cuda").to(torch.complex64), torch.ones(40, 1, device="cuda", dtype=torch.complex64)
+    for kw, pitch in (({}, L), ({"padded": True}, L + L % 2)):
+        out, x = ext.fwd(u, delta, A, one, one, None, "zoh", **kw)
+        du = ext.bwd(u, delta, A, one, one, None, dout, x, "zoh", **kw)[0]
+        assert out.stride() == du.stride() == (40 * pitch, pitch, 1)

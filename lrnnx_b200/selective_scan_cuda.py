@@ -340,19 +340,13 @@ def bwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, dout, x_, out_, dz_, de
             _shape(x_, batch, dim, n_chunks, 2 * dstate, name="x")
         du = torch.empty_like(u)
         ddelta = torch.empty_like(delta)
-        if A.is_contiguous() and A.dtype == torch.float32 and var_B and var_C and B.is_contiguous() and C.is_contiguous():
-            # two fills instead of five: the parameters' gradients, and the (larger) sums for B and C
-            n, nD, nb = A.numel(), (0 if D_ is None else dim), (0 if delta_bias_ is None else dim)
-            dA, dD, ddelta_bias = torch.zeros(n + nD + nb, dtype=torch.float32, device=u.device).split((n, nD, nb))
-            dA = dA.view(A.shape)
-            dD, ddelta_bias = (dD if nD else None), (ddelta_bias if nb else None)
-            dB, dC = torch.zeros((2, *B.shape), dtype=torch.float32, device=u.device).unbind(0)
-        else:
-            dA = torch.zeros_like(A)
-            dB = torch.zeros_like(B) if not var_B else torch.zeros_like(B, dtype=torch.float32)
-            dC = torch.zeros_like(C) if not var_C else torch.zeros_like(C, dtype=torch.float32)
-            dD = torch.zeros_like(D_) if D_ is not None else None
-            ddelta_bias = torch.zeros_like(delta_bias_) if delta_bias_ is not None else None
+        dA = torch.empty_like(A)
+        dB = torch.empty_like(B) if not var_B else torch.empty_like(B, dtype=torch.float32)
+        dC = torch.empty_like(C) if not var_C else torch.empty_like(C, dtype=torch.float32)
+        dD = torch.empty_like(D_) if D_ is not None else None
+        ddelta_bias = torch.empty_like(delta_bias_) if delta_bias_ is not None else None
+        # one launch for all the accumulators; each is a tensor of its own, which a caller may keep without the others
+        torch._foreach_zero_([t for t in (dA, dB, dC, dD, ddelta_bias) if t is not None])
         ddeltaA = torch.empty_like(deltaA_) if deltaA_ is not None else None
 
         q = _lib.struct("b200_selscan_bwd_args")()

@@ -188,3 +188,13 @@ def test_slices_of_the_backward(dim, groups, states, monkeypatch):
     size = channel - 1
     with pytest.raises(RuntimeError, match="too small"):
         ext.bwd(*args, dout, x, out, None, True, False, "mamba", **kw)
+
+
+def test_gradients_own_their_memory():
+    """A caller that keeps one gradient keeps that one alone."""
+    from lrnnx_b200.ops import selective_scan_fn
+    t, g = _make_inputs(2, 24, 16, 40, seed=3)
+    kw = dict(delta_softplus=True, discretization="mamba")
+    _, grads = _grads({k: (v.cuda() if torch.is_tensor(v) else v) for k, v in t.items()}, kw, torch.randn(2, 24, 40, generator=g).cuda(), selective_scan_fn)
+    for k, v in grads.items():
+        assert v.untyped_storage().nbytes() == v.numel() * v.element_size(), k

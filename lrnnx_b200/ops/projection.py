@@ -17,7 +17,7 @@ from .. import _lib
 
 
 def _complex_product(W, x) -> bool:
-    return (W.is_cuda and x.is_cuda and W.dtype == torch.complex64 and x.dtype == torch.complex64 and W.dim() == 2 and x.dim() == 3
+    return (W.is_cuda and W.device == x.device and W.dtype == torch.complex64 and x.dtype == torch.complex64 and W.dim() == 2 and x.dim() == 3
             and x.shape[1] == W.shape[1])
 
 
@@ -104,7 +104,7 @@ def product(W, x, conj_transpose=False, padded=False):
 
 
 def grad_supported(g, u) -> bool:
-    if not (g.is_cuda and u.is_cuda and g.dtype == torch.complex64 and u.dtype == torch.complex64):
+    if not (g.is_cuda and g.device == u.device and g.dtype == torch.complex64 and u.dtype == torch.complex64):
         return False
     if g.dim() != 3 or u.dim() != 3 or g.shape[0] != u.shape[0] or g.shape[2] != u.shape[2]:
         return False
@@ -112,7 +112,7 @@ def grad_supported(g, u) -> bool:
 
 
 def grad_fits(g, u) -> bool:
-    return (g.is_cuda and u.is_cuda and g.dtype == torch.complex64 and u.dtype == torch.complex64 and g.dim() == 3 and u.dim() == 3
+    return (g.is_cuda and g.device == u.device and g.dtype == torch.complex64 and u.dtype == torch.complex64 and g.dim() == 3 and u.dim() == 3
             and g.shape[0] == u.shape[0] and g.shape[2] == u.shape[2] and min(g.shape[1], u.shape[1]) >= 32 and g.numel() > 0)
 
 

@@ -143,6 +143,29 @@ def test_python_shims_validate_like_the_reference():
                                                torch.randn(2, 4, dtype=torch.complex64))
 
 
+def test_projections_leave_operands_of_two_devices_to_torch():
+    """torch's einsum refuses them; a kernel would read the other GPU's addresses."""
+    from lrnnx_b200.ops import projection
+
+    class Fake:
+        is_cuda, dtype = True, torch.complex64
+
+        def __init__(self, device, *shape):
+            self.device, self.shape = torch.device(device), torch.Size(shape)
+
+        def dim(self):
+            return len(self.shape)
+
+        def numel(self):
+            return self.shape.numel()
+
+    W, x, g = Fake("cuda:0", 64, 48), Fake("cuda:0", 2, 48, 99), Fake("cuda:0", 2, 64, 99)
+    assert projection.fits(W, x) and projection.grad_fits(g, x)
+    x.device = torch.device("cuda:1")
+    assert not projection.fits(W, x) and not projection.grad_fits(g, x)
+    assert not projection.supported(W, x) and not projection.grad_supported(g, x)
+
+
 def test_install_registers_extension_modules():
     import sys
     import lrnnx_b200

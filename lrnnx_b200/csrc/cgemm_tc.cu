@@ -81,7 +81,8 @@ __device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64
 }
 // The tensor core truncates a 32-bit operand to TF32, so the high part of x is what it reads from
 // the tile as it is; the low part x - trunc(x) is exact in float32 and is rounded to the nearest
-// TF32 here (the hardware would truncate it, a one-sided error that adds up over K).
+// TF32 here (the hardware would truncate it, a one-sided error that adds up over K).  Of an infinity the low part is a
+// zero: inf - inf is the canonical NaN 0x7fffffff, which the rounding carries over into -0.
 __device__ __forceinline__ float tf32_low(float v) {
   const float r = v - __uint_as_float(__float_as_uint(v) & 0xffffe000u);
   return __uint_as_float((__float_as_uint(r) + 0x1000u) & 0xffffe000u);
@@ -114,6 +115,27 @@ __device__ __forceinline__ bool wait_given_back(uint64_t *bar, int n, int slots)
 
 template <int R> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
 template <int R> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
+
+// The real (even col) or imaginary part of W x in float column `col` of the rows m0 + i whose bit is set, as a plain sum.
+__device__ __forceinline__ void plain_rows(const b200_cgemm_args &p, int mt, uint64_t set, int m0, int col, int b, float *orow) {
+  const int Kp = (p.K + KPAD - 1) / KPAD * KPAD;
+  const int64_t plane = (int64_t)mt * GM * Kp;
+  const float2 *x = reinterpret_cast<const float2 *>(p.x) + (int64_t)b * p.x_bs + (col >> 1);
+  for (; set; set &= set - 1) {
+    const int i = __ffsll((long long)set) - 1;
+    const float *w = reinterpret_cast<const float *>(p.w_planes) + (int64_t)(m0 + i) * Kp;
+    float s = 0.f;
+    for (int k0 = 0; k0 < p.K && s == s; k0 += 8) {        // a NaN stays one
+#pragma unroll
+      for (int k = k0; k < k0 + 8; ++k) {
+        const float wr = w[k] + w[plane + k], wi = w[2 * plane + k] + w[3 * plane + k];      // the planes reach to Kp
+        const float2 v = k < p.K ? x[(int64_t)k * p.x_ks] : make_float2(0.f, 0.f);
+        s = (col & 1) ? fmaf(wr, v.y, fmaf(wi, v.x, s)) : fmaf(wr, v.x, fmaf(-wi, v.y, s));
+      }
+    }
+    orow[(int64_t)i * p.out_ms * 2] = s;
+  }
+}
 
 __global__ void __launch_bounds__(NTHREADS, 1)
 cgemm_wx_kernel(const __grid_constant__ GemmMaps maps, const b200_cgemm_args p, const int mt, const int nt, const int nk) {
@@ -249,11 +271,16 @@ cgemm_wx_kernel(const __grid_constant__ GemmMaps maps, const b200_cgemm_args p, 
         const float sign = (lane & 1) ? 1.f : -1.f;
         const int rows = p.M - m0;
         const bool in = col < 2 * p.N;
+        uint64_t nan = 0;
 #pragma unroll
         for (int i = 0; i < GM / 2; ++i) {
-          const float other = __shfl_xor_sync(0xffffffffu, acc2[i], 1);
-          if (i < rows && in) orow[(int64_t)i * p.out_ms * 2] = fmaf(sign, other, acc1[i]);
+          const float other = __shfl_xor_sync(0xffffffffu, acc2[i], 1), v = fmaf(sign, other, acc1[i]);
+          if (i < rows && in) {
+            orow[(int64_t)i * p.out_ms * 2] = v;
+            if (v != v) nan |= uint64_t(1) << i;
+          }
         }
+        if (nan) plain_rows(p, mt, nan, m0, col, b, orow);
       }
     }
     if (!ok) atomicExch(&pipe.fail, 1);
@@ -286,6 +313,29 @@ struct GradMaps {
   CUtensorMap g;      // (2 L, batch M) float32, box (16, 128)
   CUtensorMap u;      // (2 L, batch N) float32, box (16, 128)
 };
+
+// This block's part (stages s_begin .. s_end) of the sum for row m and columns n, n + 32 of the output, as a plain sum, for
+// the rows m + r whose bit is set in the column's mask.
+__device__ __forceinline__ void plain_sums(const b200_cgemm_grad_args &p, uint32_t set0, uint32_t set1, int m, int n, int s_begin, int s_end) {
+  const int per_batch = (2 * p.L + GK - 1) / GK;
+  for (uint64_t set = set0 | (uint64_t)set1 << 32; set; set &= set - 1) {
+    const int i = __ffsll((long long)set) - 1, mm = m + (i & 31), nn = n + (i & 32);
+    float re = 0.f, im = 0.f;
+    for (int s = s_begin; s < s_end && (re == re || im == im); ++s) {
+      const int b = s / per_batch, l0 = s % per_batch * (GK / 2);
+      const float2 *g = reinterpret_cast<const float2 *>(p.g) + ((int64_t)b * p.M + mm) * p.g_rs + l0;
+      const float2 *u = reinterpret_cast<const float2 *>(p.u) + ((int64_t)b * p.N + nn) * p.u_rs + l0;
+#pragma unroll
+      for (int l = 0; l < GK / 2; ++l) {
+        const float2 x = l < p.L - l0 ? g[l] : make_float2(0.f, 0.f), y = l < p.L - l0 ? u[l] : make_float2(0.f, 0.f);
+        re = fmaf(x.x, y.x, fmaf(x.y, y.y, re));
+        im = fmaf(x.y, y.x, fmaf(-x.x, y.y, im));
+      }
+    }
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(reinterpret_cast<float *>(p.out) + ((int64_t)mm * p.N + nn) * 2), "f"(re), "f"(im)
+                 : "memory");
+  }
+}
 
 __global__ void __launch_bounds__(NTHREADS, 1)
 cgemm_ggh_kernel(const __grid_constant__ GradMaps maps, const b200_cgemm_grad_args p, const int stages_per_cta) {
@@ -405,8 +455,10 @@ cgemm_ggh_kernel(const __grid_constant__ GradMaps maps, const b200_cgemm_grad_ar
       // that a warp adds 32 consecutive complex elements of one row per instruction.  The stage buffers are free:
       // the last acc_full said that every MMA has read them and nothing is in flight.
       float2 *turn = reinterpret_cast<float2 *>(smem) + (size_t)(warp - 8) * 32 * 33;
+      uint32_t nan[GN / 64];
 #pragma unroll
       for (int c = 0; c < GN / 64; ++c) {
+        nan[c] = 0;
 #pragma unroll
         for (int j = 0; j < 32; ++j) turn[lane * 33 + j] = make_float2(re[c * 32 + j], im[c * 32 + j]);
         __syncwarp();
@@ -415,13 +467,16 @@ cgemm_ggh_kernel(const __grid_constant__ GradMaps maps, const b200_cgemm_grad_ar
         for (int r = 0; r < 32; ++r) {
           const float2 v = turn[r * 33 + lane];
           const int m = m0 + q * 32 + r;
-          if (m < p.M && n < p.N)
+          if (m >= p.M || n >= p.N) continue;
+          if (v.x != v.x || v.y != v.y) nan[c] |= 1u << r;
+          else
             asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(reinterpret_cast<float *>(p.out) + ((int64_t)m * p.N + n) * 2),
                          "f"(v.x), "f"(v.y)
                          : "memory");
         }
         __syncwarp();
       }
+      if (nan[0] | nan[1]) plain_sums(p, nan[0], nan[1], m0 + q * 32, n0 + h * (GN / 2) + lane, s_begin, s_begin + nk);
     }
   }
   tc_fence_before();
@@ -430,6 +485,14 @@ cgemm_ggh_kernel(const __grid_constant__ GradMaps maps, const b200_cgemm_grad_ar
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
   if (tid == 0 && pipe.fail) atomicExch(&g_cgemm_status, 6);
+}
+
+// v rounded to the nearest TF32; a NaN stays one (its bits would carry over into a zero) and what would round to
+// infinity is truncated
+__device__ __forceinline__ float tf32_high(float v) {
+  const uint32_t u = __float_as_uint(v), r = (u + 0x1000u) & 0xffffe000u;
+  if (v != v) return __uint_as_float(0x7fc00000u);
+  return __uint_as_float((r & 0x7fffffffu) == 0x7f800000u ? u & 0xffffe000u : r);
 }
 
 // Weight planes for cgemm_wx_kernel: (4, Mp, Kp) float32 = tf32(Re W), tf32(Re W - that), and the same
@@ -442,9 +505,8 @@ __global__ void cgemm_planes_kernel(const float2 *w, int M, int K, int Mp, int K
   const int m = (int)(i / Kp), k = (int)(i % Kp);
   float2 v = m < M && k < K ? w[(int64_t)m * rs + (int64_t)k * cs] : make_float2(0.f, 0.f);
   if (conj) v.y = -v.y;
-  const float rh = __uint_as_float((__float_as_uint(v.x) + 0x1000u) & 0xffffe000u);
-  const float ih = __uint_as_float((__float_as_uint(v.y) + 0x1000u) & 0xffffe000u);
-  const float rl = v.x - rh, il = v.y - ih;
+  const float rh = tf32_high(v.x), ih = tf32_high(v.y);
+  const float rl = v.x - rh, il = v.y - ih;                 // of an infinity or a NaN: the canonical NaN, which becomes -0 below
   planes[i] = rh;
   planes[MK + i] = __uint_as_float((__float_as_uint(rl) + 0x1000u) & 0xffffe000u);
   planes[2 * MK + i] = ih;
@@ -514,7 +576,10 @@ extern "C" int b200_cgemm_grad(const b200_cgemm_grad_args *args, void *stream) {
   if (pieces < 1) pieces = 1;
   const int64_t per = (total + pieces - 1) / pieces;
   const dim3 grid((unsigned)nt, (unsigned)mt, (unsigned)((total + per - 1) / per));
-  cgemm_ggh_kernel<<<grid, NTHREADS, smem, reinterpret_cast<cudaStream_t>(stream)>>>(maps, a, (int)per);
+  b200_cgemm_grad_args k = a;
+  k.g_rs = g_rs;
+  k.u_rs = u_rs;
+  cgemm_ggh_kernel<<<grid, NTHREADS, smem, reinterpret_cast<cudaStream_t>(stream)>>>(maps, k, (int)per);
   return launch_status();
 }
 

@@ -82,3 +82,41 @@ def test_the_extension_lays_its_outputs_out_as_before(L):
         out, x = ext.fwd(u, delta, A, one, one, None, "zoh", **kw)
         du = ext.bwd(u, delta, A, one, one, None, dout, x, "zoh", **kw)[0]
         assert out.stride() == du.stride() == (40 * pitch, pitch, 1)
+
+
+def _plain(spec, a, b):
+    """The complex sum as four real ones in float64: what is infinite or not a number follows from IEEE arithmetic alone."""
+    a, b = a.cpu().to(torch.complex128), b.cpu().to(torch.complex128)
+    e = lambda x, y: torch.einsum(spec, x, y)  # noqa: E731
+    return e(a.real, b.real) - e(a.imag, b.imag), e(a.real, b.imag) + e(a.imag, b.real)
+
+
+def _same_specials(got, want):
+    for x, y in zip((got.real.cpu().double(), got.imag.cpu().double()), want):
+        assert torch.equal(x.isnan(), y.isnan())
+        fin = y.isfinite()
+        assert torch.equal(x[~fin & ~y.isnan()], y[~fin & ~y.isnan()])          # infinities and their signs
+        assert bool(fin.any())
+        assert float((x - y)[fin].abs().max()) <= 1e-6 * float(y[fin].abs().max())
+
+
+@pytest.mark.parametrize("M,K,N", [(40, 47, 77), (130, 64, 129), (256, 128, 192)])
+def test_infinities_and_nans(M, K, N):
+    """An infinite or missing value in either operand reaches the outputs that depend on it, as in any float32 product, and
+    no others; a weight that is zero or exact in TF32 makes no NaN of an infinity; the largest float32 stays finite."""
+    from lrnnx_b200.ops import projection
+    g = torch.Generator().manual_seed(M)
+    inf, nan = float("inf"), (torch.zeros(1, device="cuda") / torch.zeros(1, device="cuda"))[0]       # the device's own NaN
+    W, x = _cn(g, M, K), _cn(g, 2, K, N)
+    W[:, 3] = 0.5 + 0.25j                                       # exact in TF32: their low parts are 0
+    x[0, 3, 5], x[1, 7, N - 1], x[0, 9, 20] = complex(inf, 0), complex(2, -inf), complex(nan, 1)
+    _same_specials(projection.product(W, x), _plain("mk,bkn->bmn", W, x))
+    _same_specials(projection.product(W.mH.contiguous(), x, True), _plain("mk,bkn->bmn", W, x))
+    W[11, 0], W[M - 1, 2], W[20, K - 1] = complex(inf, 1), complex(0.5, nan), 3.4028e38
+    x = 1e-30 * _cn(g, 2, K, N)
+    _same_specials(projection.product(W, x), _plain("mk,bkn->bmn", W, x))
+
+    a, b = _cn(g, 2, M, N), _cn(g, 2, K, N)
+    b[:, 1] = 1 + 0.5j
+    a[0, 3, 5], a[1, M - 1, N - 1], b[1, K - 1, 0] = complex(inf, 0), complex(1, nan), complex(0, -inf)
+    _same_specials(projection.gradient(a, b), _plain("bml,bnl->mn", a, b.conj()))

@@ -41,6 +41,7 @@ __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
 
 // Both terms of a conjugate pair share the real part dr of z - w and z - conj(w); with e1 = zi - wi, e2 = zi + wi
 //     v / (z - w) + conj(v) / (z - conj(w)) = v (dr, -e1) / (dr^2 + e1^2) + conj(v) (dr, -e2) / (dr^2 + e2^2)
@@ -79,10 +80,8 @@ __global__ void __launch_bounds__(CT) cauchy_fwd_kernel(const cf *__restrict__ v
         const float2 dd = mul2(dr, dr);
         const float2 r1 = rcp2(fma2(e1, e1, dd)), r2 = rcp2(fma2(e2, e2, dd));
         const float2 r1r = mul2(dr, r1), r1n = mul2(e1, r1), r2r = mul2(dr, r2), r2n = mul2(e2, r2);
-        ar[j] = fma2(both(t.x), r1r, fma2(both(t.y), r1n, ar[j]));
-        ar[j] = fma2(both(t.x), r2r, fma2(both(-t.y), r2n, ar[j]));
-        ai[j] = fma2(both(t.y), r1r, fma2(both(-t.x), r1n, ai[j]));
-        ai[j] = fma2(both(-t.y), r2r, fma2(both(-t.x), r2n, ai[j]));
+        ar[j] = fma2(both(t.x), add2(r1r, r2r), fma2(both(t.y), sub2(r1n, r2n), ar[j]));
+        ai[j] = fma2(both(t.y), sub2(r1r, r2r), fma2(both(-t.x), add2(r1n, r2n), ai[j]));
       }
     }
   }
@@ -187,14 +186,10 @@ __global__ void __launch_bounds__(BTT) s4_bwd_partial_kernel(const cf *__restric
         const float2 s2r = fma2(gin, r2n, mul2(gr, r2r)), s2n = fma2(gr, r2n, mul2(gi, r2r));            // s2 = (s2r, -s2n)
         b1r[k] = add2(b1r[k], add2(s1r, s2r));
         b1i[k] = add2(b1i[k], fma2(s2n, m, s1i));
-        b2r[k] = fma2(s1r, r1r, b2r[k]);
-        b2r[k] = fma2(mul2(s1i, m), r1i, b2r[k]);
-        b2r[k] = fma2(s2r, r2r, b2r[k]);
-        b2r[k] = fma2(mul2(s2n, m), r2n, b2r[k]);
-        b2i[k] = fma2(s1r, r1i, b2i[k]);
-        b2i[k] = fma2(s1i, r1r, b2i[k]);
-        const float2 c = fma2(s2r, r2n, mul2(s2n, r2r));
-        b2i[k] = fma2(c, m, b2i[k]);
+        const float2 tr = fma2(s2r, r2r, mul2(s1r, r1r)), ur = fma2(s2n, r2n, mul2(s1i, r1i));
+        const float2 ti = fma2(s1i, r1r, mul2(s1r, r1i)), ui = fma2(s2r, r2n, mul2(s2n, r2r));
+        b2r[k] = add2(b2r[k], fma2(ur, m, tr));
+        b2i[k] = add2(b2i[k], fma2(ui, m, ti));
       }
     }
 #pragma unroll

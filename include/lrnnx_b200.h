@@ -110,9 +110,8 @@ int b200_selscan_fwd(const b200_selscan_fwd_args *args, void *stream);
 
 /* Stage spacing (in steps) with which b200_selscan_fwd with these arguments (stage_h and
  * stage_len aside) would write stage_h and b200_selscan_bwd on the same problem would read it;
- * 0 if stage states are not used for this problem.  Non-zero on the shape class of the
- * state-parallel kernels with l_segments <= 1: 256, or 32 for problems of at least
- * LRNNX_B200_SL_MIN_WARPS (environment variable) tiles of 16 channels. */
+ * 0 if stage states are not used for this problem.  256 on the shape class of the
+ * state-parallel kernels with l_segments <= 1.  Any other stage_len is as good as a null stage_h. */
 int b200_selscan_stage_states(const b200_selscan_fwd_args *args);
 
 /* ------------------------------------------------------------------------

@@ -74,7 +74,7 @@ int b200_selscan_fwd(const b200_selscan_fwd_args *args, void *stream) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (selscan_seq_supported(*args)) {
     b200_selscan_fwd_args a = *args;
-    if (!stage_usable(a.stage_len)) a.stage_h = nullptr;
+    if (a.stage_len != kStage) a.stage_h = nullptr;
     return selscan_seq_fwd(a, st);
   }
   B200_REQUIRE(args->l_segments <= 1, B200_ERR_UNSUPPORTED,
@@ -87,7 +87,7 @@ int b200_selscan_stage_states(const b200_selscan_fwd_args *args) {
   if (!args || check_selscan(*args) || args->l_segments > 1) return 0;
   b200_selscan_fwd_args a = *args;
   a.stage_h = nullptr;
-  return selscan_seq_supported(a) ? selscan_seq_stage_len(a) : 0;
+  return selscan_seq_supported(a) ? kStage : 0;
 }
 
 int64_t b200_selscan_bwd_work_bytes(const b200_selscan_bwd_args *args) {
@@ -115,7 +115,7 @@ int b200_selscan_bwd(const b200_selscan_bwd_args *args, void *stream) {
   if (!selscan_seq_bwd_supported(*args)) return selscan_bwd_generic(*args, st);
   b200_selscan_bwd_args a = *args;
   // the forward's stage states start from zero: with a state entering the sequence they are not its states
-  if (!stage_usable(a.f.stage_len) || a.h_in) a.f.stage_h = nullptr;
+  if (a.f.stage_len != kStage || a.h_in) a.f.stage_h = nullptr;
   B200_REQUIRE((reinterpret_cast<uintptr_t>(a.work) & 31) == 0, B200_ERR_ALIGN, "selscan_bwd: work must be 32-byte aligned");
   if (a.work) return selscan_seq_bwd(a, a.work, a.work_bytes, st);
   void *work = nullptr;

@@ -5,10 +5,10 @@
 
 namespace b200 {
 
-constexpr int kStage = 256;       // the state-parallel backward starts its walks every so many steps
-// Spacings of stage_h that it can start them from: whole 32-step stages, of which one ends where each walk begins.
-// States of any other spacing are neither written nor read.
-inline bool stage_usable(int stage_len) { return stage_len > 0 && stage_len % 32 == 0 && kStage % stage_len == 0; }
+// Spacing of the states that the state-parallel forward leaves for the backward, which starts its own walk from them:
+// pieces of 256 steps fill the GPU wherever the rows alone do not, and closer states would only cost memory (every 32
+// steps they are as large as a 16-bit activation).  States of any other spacing are neither written nor read.
+constexpr int kStage = 256;
 
 // coverage kernels: every variant (selscan_generic.cu)
 int selscan_fwd_generic(const b200_selscan_fwd_args &a, cudaStream_t st);
@@ -16,7 +16,6 @@ int selscan_bwd_generic(const b200_selscan_bwd_args &a, cudaStream_t st);
 
 // state-parallel kernels (selscan_seq.cu, selscan_seq_bwd.cu)
 bool selscan_seq_supported(const b200_selscan_fwd_args &a);
-int selscan_seq_stage_len(const b200_selscan_fwd_args &a);
 int selscan_seq_fwd(const b200_selscan_fwd_args &a, cudaStream_t st);
 bool selscan_seq_bwd_supported(const b200_selscan_bwd_args &a);
 int64_t selscan_seq_bwd_bytes(const b200_selscan_fwd_args &f);

@@ -20,7 +20,6 @@
 // float32 call takes 90 us where the one-warp-per-row kernel that used to serve odd lengths took 1.1 ms.
 // Results match csrc/selective_scan/selective_scan.cuh:73-382 of lrnnx for this shape class.
 #include "selscan_seq.cuh"
-#include <cstdlib>
 
 namespace b200 {
 namespace {
@@ -311,16 +310,6 @@ bool selscan_seq_supported(const b200_selscan_fwd_args &a) {
   // 128-bit accesses: the states in x and stage_h
   if ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.stage_h)) & 15) return false;
   return fwd_blocks(a) < (int64_t)1 << 31;
-}
-
-// Spacing of the states that a forward call leaves for the backward, which starts its own walk from them in pieces
-// of 256 steps: that many pieces fill the GPU wherever the rows alone do not, and closer states would only cost memory
-// (every 32 steps they are as large as a 16-bit activation).  The environment variable names a number of 16-channel
-// tiles from which on a problem saves its states every 32 steps all the same.
-int selscan_seq_stage_len(const b200_selscan_fwd_args &a) {
-  const char *e = getenv("LRNNX_B200_SL_MIN_WARPS");
-  const int64_t warps = (int64_t)a.batch * ((a.dim + 15) / 16);
-  return e && warps >= atoll(e) ? 32 : kStage;
 }
 
 int selscan_seq_fwd(const b200_selscan_fwd_args &a, cudaStream_t st) {

@@ -165,12 +165,18 @@ def test_argument_errors():
         selective_scan_cuda.fwd(u.cpu(), u, A, B, B, None, None, None, None, False, "mamba")
 
 
-@pytest.fixture(params=["stream", "lanescan"])
+@pytest.fixture(params=["state-parallel", "coverage"])
 def kernel_family(request, monkeypatch):
-    """Runs a test once on each throughput-kernel family: the library picks the streaming kernels
-    (one warp per 16 channels, serial in time) when a problem has at least
-    LRNNX_B200_SL_MIN_WARPS warps of work and the lane-scan kernels otherwise."""
-    monkeypatch.setenv("LRNNX_B200_SL_MIN_WARPS", "1" if request.param == "stream" else "1000000000")
+    """Runs a test once on the state-parallel kernels and once on the coverage kernels, which take a call
+    whose checkpoints are not 16-byte aligned: the tensor that holds them starts one element off."""
+    if request.param == "coverage":
+        empty = torch.empty
+
+        def shifted(*size, **kw):
+            if len(size) == 1 and isinstance(size[0], int) and kw.get("dtype") == torch.float32:
+                return empty(size[0] + 1, **kw)[1:]
+            return empty(*size, **kw)
+        monkeypatch.setattr(torch, "empty", shifted)
     return request.param
 
 
@@ -178,9 +184,8 @@ def kernel_family(request, monkeypatch):
 @pytest.mark.parametrize("dtype,groups", [(torch.float32, 1), (torch.float32, 2), (torch.bfloat16, 1),
                                           (torch.float16, 2)])
 def test_throughput_kernel_shape_class(L, dtype, groups, kernel_family):
-    """Shapes served by the packed-fp32 throughput kernels (real A, mamba, variable B/C, dstate 16,
-    channel count a multiple of 16 per group, L a multiple of 8): one and several stages, a ragged
-    last stage, and a 2048-step checkpoint boundary; on both kernel families."""
+    """Real A, mamba, variable B/C, dstate 16: one and several stages, a ragged last stage, and a
+    2048-step checkpoint boundary; on both kernel families."""
     t, g = _make_inputs(2, 32 * groups, 16, L, seed=L, dtype=dtype, groups=groups)
     if dtype == torch.float32:
         _oracle_vs_gpu(t, g, "mamba", RTOL32, ATOL32, GRAD_RTOL32, GRAD_ATOL32)
@@ -217,9 +222,8 @@ def test_throughput_kernel_optional_operands(with_z, with_D, with_bias, softplus
         assert_close(a.cpu(), b, rtol=GRAD_RTOL32, atol_scale=GRAD_ATOL32, name=f"d{k}")
 
 
-def test_streaming_kernel_many_tiles():
-    """Enough rows that the library picks the streaming kernels by itself (at least two warps of
-    work per SM): 4 x 1280 channels in 2 groups, two stages plus a ragged one."""
+def test_many_tiles():
+    """More than one thread block per SM: 4 x 1280 channels in 2 groups, two stages plus a ragged one."""
     t, g = _make_inputs(4, 1280, 16, 72, seed=12, groups=2)
     _oracle_vs_gpu(t, g, "mamba", RTOL32, ATOL32, GRAD_RTOL32, GRAD_ATOL32)
 
@@ -237,8 +241,8 @@ def test_throughput_kernel_checkpoints(kernel_family):
 
 
 @pytest.mark.parametrize("dtype,L", [(torch.float32, 4360), (torch.bfloat16, 2048), (torch.bfloat16, 520)])
-def test_backward_with_and_without_saved_stage_states(dtype, L, kernel_family):
-    """The forward call of the throughput kernels leaves the state at every stage boundary
+def test_backward_with_and_without_saved_stage_states(dtype, L):
+    """The forward call of the state-parallel kernels leaves the state at every stage boundary
     behind the checkpoints of x; the backward call uses them when it is handed that x and
     recomputes them when it is handed a copy, or a tensor of the same size that did not come from
     fwd().  All must give the same gradients."""
@@ -248,7 +252,7 @@ def test_backward_with_and_without_saved_stage_states(dtype, L, kernel_family):
     args = (cu["u"], cu["delta"], cu["A"], cu["B"], cu["C"], cu["D"], cu["z"], cu["delta_bias"], None)
     out, x, out_z = ext.fwd(*args, True, "mamba")
     ptr, stage_len = ext._stage_states_of(x, 2, 16, L, 16)
-    assert ptr is not None and stage_len == (32 if kernel_family == "stream" else 256)
+    assert ptr is not None and stage_len == 256
     assert ext._stage_states_of(x.clone(), 2, 16, L, 16) == (None, 0)
     # a caller-built x whose allocation happens to have the same size is not mistaken for one made by fwd()
     fake = torch.empty(x.untyped_storage().nbytes() // 4, device="cuda")[: x.numel()].view_as(x).copy_(x)

@@ -1,7 +1,9 @@
 """The state-parallel selective-scan kernels where their tilings can go wrong: channel counts that leave a
 warp (8 channels), a thread block (32) or a group partly empty, lengths around the 4-step blocks, the
 32-step stages, the 128-step windows, the 256-step pieces and the 2048-step checkpoints, rows that are not
-16-byte aligned, and the three ways the backward gets its states and its workspace."""
+16-byte aligned, orders of the strides, entering states and adjoints, segments of the sequence, and the ways the
+backward gets its states and its workspace.  Against the oracle, or against the coverage kernels, which take any
+call whose checkpoints are not 16-byte aligned."""
 from __future__ import annotations
 
 import pytest
@@ -198,3 +200,66 @@ def test_gradients_own_their_memory():
     _, grads = _grads({k: (v.cuda() if torch.is_tensor(v) else v) for k, v in t.items()}, kw, torch.randn(2, 24, 40, generator=g).cuda(), selective_scan_fn)
     for k, v in grads.items():
         assert v.untyped_storage().nbytes() == v.numel() * v.element_size(), k
+
+
+def _off_alignment(x):
+    """A copy of x that the state-parallel kernels do not take."""
+    y = torch.empty(x.numel() + 1, dtype=x.dtype, device=x.device)[1:].view(x.shape)
+    return y.copy_(x)
+
+
+@pytest.mark.parametrize("batch,dim,groups,L", [(2, 20, 1, 333), (1, 36, 2, 2049), (3, 9, 3, 130)])
+@pytest.mark.parametrize("layout", ["dense", "channel-major", "unaligned"])
+def test_entering_state_and_adjoint_against_the_coverage_kernels(batch, dim, groups, L, layout):
+    from lrnnx_b200 import selective_scan_cuda as ext
+    t, g = _make_inputs(batch, dim, 16, L, seed=L, groups=groups)
+    c = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in t.items()}
+    dout = torch.randn(batch, dim, L, generator=g).cuda()
+
+    def lay(v):
+        if layout == "channel-major":
+            return v.transpose(0, 1).contiguous().transpose(0, 1)
+        wide = torch.full((*v.shape[:-1], L + 5), float("nan"), device="cuda")
+        return wide[..., 3:3 + L].copy_(v) if layout == "unaligned" else v
+
+    for k in ("u", "delta", "z", "B", "C"):
+        c[k] = lay(c[k])
+    dout = lay(dout)
+    args = (c["u"], c["delta"], c["A"], c["B"], c["C"], c["D"], c["z"], c["delta_bias"], None)
+    out, x, _ = ext.fwd(*args, True, "mamba")
+    for kw in ({}, {"h_in"}, {"q_in"}, {"h_in", "q_in"}):
+        kw = {k: torch.randn(batch, dim, 16, generator=g).cuda() for k in sorted(kw)}
+        got = ext.bwd(*args, dout, x, out, None, True, False, "mamba", **kw)
+        want = ext.bwd(*args, dout, _off_alignment(x), out, None, True, False, "mamba", **kw)
+        for i, (a, b) in enumerate(zip(got, want)):
+            assert_close(a.cpu(), b.cpu(), rtol=GRAD_RTOL32, atol_scale=GRAD_ATOL32, name=f"{sorted(kw)} gradient {i}")
+
+
+@pytest.mark.parametrize("dim,groups,L", [(20, 1, 5 * 2048 + 131), (42, 2, 4 * 2048 + 1), (33, 3, 4 * 2048)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_segments_at_odd_sizes(dim, groups, L, offset):
+    """A float32 call of few rows is cut into segments at any length, channel count and alignment: outputs, checkpoints
+    and gradients against the same call in one piece."""
+    from lrnnx_b200 import selective_scan_cuda as ext
+    t, g = _make_inputs(1, dim, 16, L, seed=L, groups=groups)
+    c = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in t.items()}
+    for k in ("u", "delta", "z", "B", "C"):
+        c[k] = torch.full((*c[k].shape[:-1], L + 3), float("nan"), device="cuda")[..., offset:offset + L].copy_(c[k])
+    args = (c["u"], c["delta"], c["A"], c["B"], c["C"], c["D"], c["z"], c["delta_bias"], None)
+    dout = torch.randn(1, dim, L, generator=g).cuda()
+    rule = ext._segments_for
+    seen = []
+
+    def run(S):
+        ext._segments_for = lambda *a: seen.append(rule(*a)) or (seen[-1] if S is None else S)
+        try:
+            out, x, out_z = ext.fwd(*args, True, "mamba")
+        finally:
+            ext._segments_for = rule
+        return [out, out_z, x] + ext.bwd(*args, dout, x, out, None, True, False, "mamba")
+
+    got, want = run(None), run(1)
+    assert seen[0] > 1
+    for i, (a, b) in enumerate(zip(got, want)):
+        grad = i > 2
+        assert_close(a.cpu(), b.cpu(), rtol=GRAD_RTOL32 if grad else RTOL32, atol_scale=GRAD_ATOL32 if grad else ATOL32, name=f"result {i}")

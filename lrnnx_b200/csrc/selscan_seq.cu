@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(FW * 32, 3) selscan_seq_fwd_kernel(const b200_
     const float *A = reinterpret_cast<const float *>(p.A) + (int64_t)(dl + min(c, max(nch - 1, 0))) * p.A_ds;
 #pragma unroll
     for (int j = 0; j < 2; ++j)
-      A2[j] = make_float2(A[(int64_t)(QS * q + 2 * j) * p.A_ns] * kLog2e, A[(int64_t)(QS * q + 2 * j + 1) * p.A_ns] * kLog2e);
+      A2[j] = make_float2(decay2(A[(int64_t)(QS * q + 2 * j) * p.A_ns]), decay2(A[(int64_t)(QS * q + 2 * j + 1) * p.A_ns]));
   }
   float bias[QCH], Dv[QCH], cs[QCH];
 #pragma unroll

@@ -40,6 +40,13 @@ template <> __device__ __forceinline__ float from_f<float>(float v) { return v; 
 template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 template <> __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half_rn(v); }
 
+// A in units of the binary logarithm.  The steps past the end have a step size of 0 and have to be neutral whatever A is:
+// an infinite decay is the largest finite one here (0 times infinity is NaN).
+__device__ __forceinline__ float decay2(float A) {
+  const float v = A * kLog2e;
+  return v < -3.402823466e38f ? -3.402823466e38f : v;
+}
+
 // softplus with the reference's pass-through above 20 (selective_scan.cuh:172-174) on two SFU
 // operations, and e = exp(x) for its derivative.  log1p(e) is a degree-5 series for e < 1/32
 // (relative error < 1e-8) and log(1 + e) above, where the absolute error of the SFU's logarithm

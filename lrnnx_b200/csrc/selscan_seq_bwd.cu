@@ -162,7 +162,7 @@ __device__ __forceinline__ void seq_walk(const b200_selscan_bwd_args &a, const S
     const float *A = reinterpret_cast<const float *>(p.A) + (int64_t)(dl + min(c, max(nch - 1, 0))) * p.A_ds;
 #pragma unroll
     for (int j = 0; j < 2; ++j)
-      A2[j] = make_float2(A[(int64_t)(QS * q + 2 * j) * p.A_ns] * kLog2e, A[(int64_t)(QS * q + 2 * j + 1) * p.A_ns] * kLog2e);
+      A2[j] = make_float2(decay2(A[(int64_t)(QS * q + 2 * j) * p.A_ns]), decay2(A[(int64_t)(QS * q + 2 * j + 1) * p.A_ns]));
   }
   float bias[QCH];
 #pragma unroll
@@ -393,7 +393,7 @@ selscan_seq_bwd_kernel(const b200_selscan_bwd_args a, const float4 *__restrict__
     rbias = bp && i + warp < i_end ? bp[g * cpg + i + warp] : 0.f;
     rD = Dvp && i + warp < i_end ? Dvp[g * cpg + i + warp] : 0.f;
     if (tid < BW * QN && i + tid / QN < i_end)
-      rA = reinterpret_cast<const float *>(p.A)[(int64_t)(g * cpg + i + tid / QN) * p.A_ds + (int64_t)(tid % QN) * p.A_ns] * kLog2e;
+      rA = decay2(reinterpret_cast<const float *>(p.A)[(int64_t)(g * cpg + i + tid / QN) * p.A_ds + (int64_t)(tid % QN) * p.A_ns]);
   };
   auto prep = [&](int i, int buf) {
     const int n = i + warp < i_end ? left : 0;

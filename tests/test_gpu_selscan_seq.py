@@ -263,3 +263,21 @@ def test_segments_at_odd_sizes(dim, groups, L, offset):
     for i, (a, b) in enumerate(zip(got, want)):
         grad = i > 2
         assert_close(a.cpu(), b.cpu(), rtol=GRAD_RTOL32 if grad else RTOL32, atol_scale=GRAD_ATOL32 if grad else ATOL32, name=f"result {i}")
+
+
+@pytest.mark.parametrize("L", [32, 37, 300])
+def test_infinite_decay(L):
+    """A state whose A is minus infinity forgets everything at each step, and is no NaN past the end of a ragged sequence.
+    (ddelta and dA have the factor A a h, infinity times 0, in them.)"""
+    from lrnnx_b200.ops import selective_scan_fn
+    t, g = _make_inputs(2, 20, 16, L, seed=L)
+    t["A"][:, 3], t["A"][5] = float("-inf"), -3e38
+    kw = dict(delta_softplus=True, discretization="mamba")
+    gout = torch.randn(2, 20, L, generator=g)
+    out_c, gc = _grads(t, kw, gout, O.selective_scan_oracle)
+    dev = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in t.items()}
+    out_g, gg = _grads(dev, kw, gout.cuda(), selective_scan_fn)
+    last_c, last_g = (fn(**x, **kw, return_last_state=True)[1] for fn, x in ((O.selective_scan_oracle, t), (selective_scan_fn, dev)))
+    for name, a, b in [("out", out_g, out_c), ("last state", last_g, last_c)] + [(k, gg[k], gc[k]) for k in ("u", "B", "C", "D", "z")]:
+        assert bool(b.isfinite().all())
+        assert_close(a.cpu(), b, rtol=GRAD_RTOL32, atol_scale=GRAD_ATOL32, name=name)

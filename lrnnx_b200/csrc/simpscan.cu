@@ -375,6 +375,16 @@ __device__ __forceinline__ void tensor_s2g(const CUtensorMap *map, int row, cons
                : "memory");
 }
 
+// Between a warp's shared-memory loads of a slice and the bulk copy that refills it.  __syncwarp alone orders them among the
+// lanes, but not before the asynchronous proxy: with bank conflicts (the linear layout of a ragged tile) and operands in
+// the L2, the copy overtook loads that still waited in the queue, and the gradient of the step sizes was made from the next
+// tile's states.  The proxy fence is the documented order; the vote on `bits`, a mix of all values loaded, is only taken
+// when they are there.  never_zero: what the compiler does not know not to be zero.  Always false.
+__device__ __forceinline__ bool before_refill(uint32_t bits, int never_zero) {
+  fence_proxy_async();
+  return __any_sync(0xffffffffu, ((bits ^ 0x9e3779b9u) | (uint32_t)never_zero) == 0u);
+}
+
 constexpr int BT = 256;               // threads per CTA
 constexpr int BI = 8;                 // timesteps per thread (BT*BI = 2048 = one checkpoint chunk)
 constexpr int BWARPS = BT / 32;
@@ -577,7 +587,12 @@ simpscan_bwd_kernel(const b200_simpscan_args p, const __grid_constant__ TmaMaps 
       }
     }
     // the warp's slice now lives in registers: refill it with the stream item two steps ahead
-    __syncwarp();
+    uint32_t bits = 0;
+#pragma unroll
+    for (int i = 0; i < BI; i += 2) bits ^= __float_as_uint(u[i].re) ^ __float_as_uint(dy[i].re);
+#pragma unroll
+    for (int i = 0; i < BI; i += 4) bits ^= __float_as_uint(dl[i]) ^ __float_as_uint(dAv[i]) << 1;
+    failed |= before_refill(bits, p.dstate);
     if (lane == 0) issue();
     bool same_step = true;
 #pragma unroll
@@ -1039,7 +1054,10 @@ simpscan_bwd_h_kernel(const b200_simpscan_args p, const __grid_constant__ TmaMap
     }
     // the read-only slices sit in registers: refill them at once; the other overwritten buffer
     // first has to be read out by the stores of the previous item
-    __syncwarp();
+    uint32_t bits = 0;
+#pragma unroll
+    for (int i = 0; i < BI; i += 2) bits ^= __float_as_uint(dy[i].re) ^ __float_as_uint(h[i].re);
+    failed |= before_refill(bits, p.dstate);
     if (lane == 0) {
       issue(1);
       if (stores_pending) bulk_wait_read<0>();

@@ -239,3 +239,24 @@ def test_single_state_backward_with_nontrivial_B_C(disc, with_dA):
                          name=f"{name} (out_={'given' if out_arg is not None else 'None'})")
     for name, a, b in zip(names, *results):
         assert_close(a.cpu(), b.cpu(), rtol=GRTOL, atol_scale=GATOL, name=f"{name}: the two backward kernels")
+
+
+@pytest.mark.parametrize("batch,P,H,L", [(6, 72, 40, 1600), (5, 120, 64, 1408)])
+def test_ragged_tiles_of_the_backward_are_read_before_they_are_refilled(batch, P, H, L):
+    """Rows of one full and one ragged tile, operands fresh from the kernels before: every pass gives the same gradient of
+    the step sizes (without a wait a tenth of the passes, or more, took states of the next tile for some steps)."""
+    from lrnnx_b200.ops import simplified_scan_fn
+    g = torch.Generator(device="cuda").manual_seed(29)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    A = torch.log(torch.polar(0.9 + 0.099 * torch.rand(P, generator=g, device="cuda"), torch.rand(P, generator=g, device="cuda")))
+    c = lambda *s: torch.complex(r(*s), r(*s))
+    t = [c(batch, H, L), torch.ones(batch, P, L, device="cuda"), A, c(P, H) / H ** 0.5, c(H, P) / P ** 0.5]
+    gout = c(batch, H, L)
+
+    def run():
+        leaves = [v.detach().requires_grad_(True) for v in t]
+        return torch.autograd.grad(simplified_scan_fn(*leaves, discretization="dirac"), leaves[1], gout)[0]
+
+    first = run()
+    for _ in range(200):
+        assert torch.equal(run(), first)

@@ -19,9 +19,11 @@
 // grows with the length of the chain (4e-6 of the result at K = 512).  So an accumulator lives for
 // two stages (32 floats of K) only: in each the small products go in first, then two large ones, and
 // the sums of a chain are added up in registers, rounded to nearest, by warps of their own.  Two sets
-// of accumulators alternate, so the next chain's products do not wait.  Error against 64 bits 2e-7,
-// whatever K (a float32 cuBLAS cgemm: 4e-7 at K = 512).  Chains of one stage would be 1.4e-7 and 10 %
-// slower, chains of the whole K 25 times less exact and no faster.
+// of accumulators alternate, so the next chain's products do not wait.  What truncation takes on average is
+// given back (a share of 1.3e-7 or less, see below): an error to one side adds up over the scan that follows,
+// and sums of positive terms only lose twice that.  Error against 64 bits 1.7e-7 at K = 96, 2.0e-7 at
+// K = 1024 (a float32 cuBLAS cgemm with a real x: 1.8e-7 and 4.1e-7).  Chains of one stage would be 10 %
+// slower, chains of the whole K 20 times less exact and no faster.
 //
 // Persistent thread blocks take 128 x 64-complex output tiles in turn: warp 0 issues the TMA loads
 // (64-byte swizzled weight tiles, 4-stage ring on mbarriers), warp 1 allocates 512 TMEM columns and
@@ -31,7 +33,8 @@
 // N = 128 (180 -> 160 us at 8 x 256 x 512 x 4096), and a TMEM lane is a float column of X, so
 // the stores are coalesced.  Sizes are free: the weight planes are padded with zeros to the tiles, the
 // tensor maps fill with zeros past K and N, and the stores stop at M and N; only the row pitch of x has to
-// be a multiple of 16 bytes.  Every mbarrier wait is bounded; an expired wait sets the status word, skips
+// be a multiple of 16 bytes.  The split of an infinity is no sum (infinity times a zero or opposite low part is
+// NaN): outputs that come out as NaN are formed once more by the plain complex sum.  Every mbarrier wait is bounded; an expired wait sets the status word, skips
 // the stores and still frees the TMEM.
 #include "common.cuh"
 #include "dispatch.h"
@@ -54,6 +57,13 @@ constexpr int TILE = GM * GK * 4;     // 8 KB: a weight-plane tile; an activatio
 constexpr int STAGE_BYTES = 6 * TILE; // Re hi, Re lo, Im hi, Im lo, X hi, X lo
 constexpr int TX_BYTES = 5 * TILE;    // what the TMA delivers per stage (X lo is produced in place)
 constexpr int PS = 2;                 // stages per accumulation chain
+// Below this K the small products of both stages of a chain go in before the large ones of either: error 1.4e-7
+// instead of 1.8e-7 (of a float32 cuBLAS product with a real x at K = 64 and 96), for up to 4 % more time.
+constexpr int SHORT_K = 160;
+// What truncation takes from a chain, as a share of a sum of random signs (measured against 64 bits, the same at all
+// sizes); the weights' low planes are that much larger, the gradient's sums are scaled
+__host__ __device__ constexpr float lost(int K) { return K < SHORT_K ? 4.3e-8f : 1.3e-7f; }
+constexpr float kLostGrad = 2.3e-7f;  // with what the product of two truncated low parts would have added
 constexpr int NTHREADS = 512;
 constexpr int TMEM_COLS = 512;        // two sets of two 128-column accumulators
 constexpr uint32_t WAIT_LIMIT = 1u << 24;
@@ -93,6 +103,7 @@ struct Pipe {
   uint64_t acc_full[2], acc_empty[2];                          // accumulator set complete / read
   uint32_t tmem_base;
   int fail;
+  int nan;                                                     // some output came out as NaN
 };
 __device__ __forceinline__ void pipe_init(Pipe &p, int sum_warps) {
   for (int s = 0; s < NSTAGE; ++s) {
@@ -105,6 +116,7 @@ __device__ __forceinline__ void pipe_init(Pipe &p, int sum_warps) {
     mbar_init(&p.acc_empty[s], sum_warps);
   }
   p.fail = 0;
+  p.nan = 0;
   mbar_fence_init();
   fence_proxy_async();
 }
@@ -116,13 +128,16 @@ __device__ __forceinline__ bool wait_given_back(uint64_t *bar, int n, int slots)
 template <int R> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
 template <int R> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
 
-// The real (even col) or imaginary part of W x in float column `col` of the rows m0 + i whose bit is set, as a plain sum.
-__device__ __forceinline__ void plain_rows(const b200_cgemm_args &p, int mt, uint64_t set, int m0, int col, int b, float *orow) {
-  const int Kp = (p.K + KPAD - 1) / KPAD * KPAD;
+// The outputs that a thread has stored as NaN in float column `col` of the GM / 2 rows from m0 on, as plain sums.
+__device__ __forceinline__ void plain_tile(const b200_cgemm_args &p, int mt, int m0, int col, int b) {
+  if (col >= 2 * p.N) return;
+  const int Kp = (p.K + KPAD - 1) / KPAD * KPAD, rows = min(p.M - m0, GM / 2);
   const int64_t plane = (int64_t)mt * GM * Kp;
   const float2 *x = reinterpret_cast<const float2 *>(p.x) + (int64_t)b * p.x_bs + (col >> 1);
-  for (; set; set &= set - 1) {
-    const int i = __ffsll((long long)set) - 1;
+  float *orow = reinterpret_cast<float *>(p.out) + ((int64_t)b * p.out_bs + (int64_t)m0 * p.out_ms) * 2 + col;
+  for (int i = 0; i < rows; ++i) {
+    const float was = orow[(int64_t)i * p.out_ms * 2];
+    if (was == was) continue;
     const float *w = reinterpret_cast<const float *>(p.w_planes) + (int64_t)(m0 + i) * Kp;
     float s = 0.f;
     for (int k0 = 0; k0 < p.K && s == s; k0 += 8) {        // a NaN stays one
@@ -184,29 +199,37 @@ cgemm_wx_kernel(const __grid_constant__ GemmMaps maps, const b200_cgemm_args p, 
     // ------------------------------------------------------------------ MMA issuer
       int g = 0, ch = 0;                       // stages, chains so far
       bool ok = true;
+      const bool small_first = p.K < SHORT_K;
       for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-        for (int ks = 0; ks < nk; ++ks, ++g) {
-          const int s = g % NSTAGE;
-          const uint32_t ph = (g / NSTAGE) & 1;
+        for (int ks = 0; ks < nk && ok; ks += PS, ++ch) {
+          const int n = min(PS, nk - ks);       // stages of this chain
           const uint32_t d = tmem_base + (ch & 1) * 2 * GN;       // columns: 128 of Re(W) X', 128 of Im(W) X'
-          if (!mbar_wait(&pipe.full[s], ph, WAIT_LIMIT) || !mbar_wait(&pipe.lo_ready[s], ph, WAIT_LIMIT) ||
-              (ks % PS == 0 && !wait_given_back(&pipe.acc_empty[ch & 1], ch, 2))) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t st = smem_u32(smem + (size_t)s * STAGE_BYTES);
-          // the small products first: what is truncated while they add up is small as well
+          const auto large = [&](int s) {
+            const uint32_t st = smem_u32(smem + (size_t)s * STAGE_BYTES);
 #pragma unroll
-          for (int kk = 0; kk < GK / 8; ++kk) {
-            const uint64_t xh = x_desc(st + 4 * TILE + kk * 1024), xl = x_desc(st + 5 * TILE + kk * 1024);
-            mma_tf32(d, xl, k_desc(st + 0 * TILE + kk * 32), kk > 0 || ks % PS != 0 ? 1u : 0u);
-            mma_tf32(d, xh, k_desc(st + 2 * TILE + kk * 32), 1u);
-          }
+            for (int kk = 0; kk < GK / 8; ++kk) mma_tf32(d, x_desc(st + 4 * TILE + kk * 1024), k_desc(st + 0 * TILE + kk * 32), 1u);
+            mma_commit(&pipe.empty[s]);         // the stage may be refilled once these MMAs have read it
+          };
+          if (!wait_given_back(&pipe.acc_empty[ch & 1], ch, 2)) { ok = false; break; }
+          for (int i = 0; i < n; ++i) {
+            const int s = (g + i) % NSTAGE;
+            const uint32_t ph = ((g + i) / NSTAGE) & 1;
+            if (!mbar_wait(&pipe.full[s], ph, WAIT_LIMIT) || !mbar_wait(&pipe.lo_ready[s], ph, WAIT_LIMIT)) { ok = false; break; }
+            tc_fence_after();
+            // the small products first: what is truncated while they add up is small as well
+            const uint32_t st = smem_u32(smem + (size_t)s * STAGE_BYTES);
 #pragma unroll
-          for (int kk = 0; kk < GK / 8; ++kk) mma_tf32(d, x_desc(st + 4 * TILE + kk * 1024), k_desc(st + 0 * TILE + kk * 32), 1u);
-          mma_commit(&pipe.empty[s]);           // the stage may be refilled once these MMAs have read it
-          if (ks % PS == PS - 1 || ks == nk - 1) {
-            mma_commit(&pipe.acc_full[ch & 1]);
-            ++ch;
+            for (int kk = 0; kk < GK / 8; ++kk) {
+              mma_tf32(d, x_desc(st + 5 * TILE + kk * 1024), k_desc(st + 0 * TILE + kk * 32), kk > 0 || i > 0 ? 1u : 0u);
+              mma_tf32(d, x_desc(st + 4 * TILE + kk * 1024), k_desc(st + 2 * TILE + kk * 32), 1u);
+            }
+            if (!small_first) large(s);
           }
+          if (!ok) break;
+          if (small_first)
+            for (int i = 0; i < n; ++i) large((g + i) % NSTAGE);
+          g += n;
+          mma_commit(&pipe.acc_full[ch & 1]);
         }
       }
       if (!ok) atomicExch(&pipe.fail, 1);
@@ -271,19 +294,20 @@ cgemm_wx_kernel(const __grid_constant__ GemmMaps maps, const b200_cgemm_args p, 
         const float sign = (lane & 1) ? 1.f : -1.f;
         const int rows = p.M - m0;
         const bool in = col < 2 * p.N;
-        uint64_t nan = 0;
+        float any = 0.f;                                // NaN if an output is (or infinities of both signs are among them)
 #pragma unroll
         for (int i = 0; i < GM / 2; ++i) {
           const float other = __shfl_xor_sync(0xffffffffu, acc2[i], 1), v = fmaf(sign, other, acc1[i]);
-          if (i < rows && in) {
-            orow[(int64_t)i * p.out_ms * 2] = v;
-            if (v != v) nan |= uint64_t(1) << i;
-          }
+          any += v;
+          if (i < rows && in) orow[(int64_t)i * p.out_ms * 2] = v;
         }
-        if (nan) plain_rows(p, mt, nan, m0, col, b, orow);
+        if (any != any) *(volatile int *)&pipe.nan = 1;
       }
     }
     if (!ok) atomicExch(&pipe.fail, 1);
+    if (*(volatile int *)&pipe.nan && ok)               // after all the tiles, where it takes no registers from them
+      for (int t = blockIdx.x; t < tiles; t += gridDim.x)
+        plain_tile(p, mt, t % mt * GM + h * (GM / 2), t / mt % nt * GN + q * 32 + lane, t / (mt * nt));
   }
   tc_fence_before();
   __syncthreads();
@@ -460,7 +484,8 @@ cgemm_ggh_kernel(const __grid_constant__ GradMaps maps, const b200_cgemm_grad_ar
       for (int c = 0; c < GN / 64; ++c) {
         nan[c] = 0;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) turn[lane * 33 + j] = make_float2(re[c * 32 + j], im[c * 32 + j]);
+        for (int j = 0; j < 32; ++j) turn[lane * 33 + j] =
+            make_float2(fmaf(re[c * 32 + j], kLostGrad, re[c * 32 + j]), fmaf(im[c * 32 + j], kLostGrad, im[c * 32 + j]));
         __syncwarp();
         const int n = n0 + h * (GN / 2) + c * 32 + lane;
 #pragma unroll 4
@@ -506,7 +531,8 @@ __global__ void cgemm_planes_kernel(const float2 *w, int M, int K, int Mp, int K
   float2 v = m < M && k < K ? w[(int64_t)m * rs + (int64_t)k * cs] : make_float2(0.f, 0.f);
   if (conj) v.y = -v.y;
   const float rh = tf32_high(v.x), ih = tf32_high(v.y);
-  const float rl = v.x - rh, il = v.y - ih;                 // of an infinity or a NaN: the canonical NaN, which becomes -0 below
+  // of an infinity or a NaN: the canonical NaN, which becomes -0 below
+  const float rl = fmaf(lost(K), v.x, v.x - rh), il = fmaf(lost(K), v.y, v.y - ih);
   planes[i] = rh;
   planes[MK + i] = __uint_as_float((__float_as_uint(rl) + 0x1000u) & 0xffffe000u);
   planes[2 * MK + i] = ih;

@@ -21,12 +21,14 @@ from . import projection
 _VALID = ("bilinear", "zoh", "dirac")
 
 
-def _proj(W, x, conj_transpose=False, padded=False):
-    """W x (or W^H x) per batch: the tensor-core kernel, or an einsum for very small products."""
-    Wm = W.conj().transpose(0, 1) if conj_transpose else W
-    if projection.fits(Wm, x):
+def _proj(W, x, conj_transpose=False, padded=False, kernel=None):
+    """W x (or W^H x) per batch: the tensor-core kernel, or an einsum for very small products (``kernel``: which, where the
+    caller has asked ``projection.fits`` already)."""
+    if kernel is None:
+        kernel = projection.fits(W.t() if conj_transpose else W, x)
+    if kernel:
         return projection.product(W, x, conj_transpose, padded)
-    return torch.einsum("mk,bkn->bmn", Wm, x)
+    return torch.einsum("mk,bkn->bmn", W.conj().transpose(0, 1) if conj_transpose else W, x)
 
 
 def _wgrad(g, u):
@@ -37,8 +39,9 @@ def _wgrad(g, u):
 
 
 def _rows(x, W):
-    """x with rows that the projection kernels read in place, where they will be used with W."""
-    return projection.rows(x) if x.is_complex() and projection.fits(W, x) else x
+    """x with rows that the projection kernels read in place, and whether they will be used with W."""
+    kernel = x.is_complex() and projection.fits(W, x)
+    return (projection.rows(x) if kernel else x), kernel
 
 
 def _kernel_A(A):
@@ -59,9 +62,9 @@ class SimplifiedScanFn(torch.autograd.Function):
         dstate = A_k.shape[1]
         Bu = _proj(B, u, padded=True)
         ident = torch.ones(P, dstate, dtype=A.dtype, device=A.device)
-        out, xs = simplified_scan_cuda.fwd(Bu, delta, A_k, ident, ident, deltaA, discretization,
-                                           padded=projection.fits(C, Bu))
-        y = _proj(C, out)
+        kernel = projection.fits(C, Bu)
+        out, xs = simplified_scan_cuda.fwd(Bu, delta, A_k, ident, ident, deltaA, discretization, padded=kernel)
+        y = _proj(C, out, kernel=kernel)
         ctx.discretization = discretization
         ctx.has_deltaA = deltaA is not None
         ctx.A_was_1d = A.dim() == 1
@@ -74,17 +77,19 @@ class SimplifiedScanFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout, *args):
         u, delta, A_k, B, C, Bu, out, xs, ident, deltaA = ctx.saved_tensors
-        dout, u = _rows(dout, C.t()), _rows(u, B)
-        dx_out = _proj(C, dout, conj_transpose=True, padded=True)
+        dout, kernel = _rows(dout, C.t())
+        u, _ = _rows(u, B)
+        dx_out = _proj(C, dout, conj_transpose=True, padded=True, kernel=kernel)
         dC = _wgrad(dout, out)
         if dx_out.stride(-1) != 1:
             dx_out = dx_out.contiguous()
+        kernel = projection.fits(B.t(), Bu)
         res = simplified_scan_cuda.bwd(Bu, delta, A_k, ident, ident, deltaA, dx_out, xs, ctx.discretization,
                                       need_dB_dC=False, out_=out if out.stride(-1) == 1 else None,
-                                      padded=projection.fits(B.t(), Bu))
+                                      padded=kernel)
         dBu, ddelta, dA = res[0], res[1], res[2]
         ddeltaA = res[5] if ctx.has_deltaA else None
-        du = _proj(B, dBu, conj_transpose=True)
+        du = _proj(B, dBu, conj_transpose=True, kernel=kernel)
         dB = _wgrad(dBu, u)
         if ctx.A_was_1d:
             dA = dA.squeeze(-1)
@@ -113,9 +118,9 @@ class S5InnerFn(torch.autograd.Function):
         dstate = A_k.shape[1]
         Bu = _proj(B, u, padded=True)
         ident = torch.ones(P, dstate, dtype=A.dtype, device=A.device)
-        scan_out, xs = simplified_scan_cuda.fwd(Bu, delta, A_k, ident, ident, deltaA, discretization,
-                                                padded=projection.fits(C, Bu))
-        y_complex = _proj(C, scan_out)
+        kernel = projection.fits(C, Bu)
+        scan_out, xs = simplified_scan_cuda.fwd(Bu, delta, A_k, ident, ident, deltaA, discretization, padded=kernel)
+        y_complex = _proj(C, scan_out, kernel=kernel)
         y_real = 2 * y_complex.real if conj_sym else y_complex.real
         u_real = u.real if u.is_complex() else u
         y = y_real + D.unsqueeze(0).unsqueeze(-1) * u_real
@@ -133,17 +138,19 @@ class S5InnerFn(torch.autograd.Function):
         du_skip = D.unsqueeze(0).unsqueeze(-1) * dout
         scale = 2.0 if ctx.conj_sym else 1.0
         dy_complex = torch.complex(scale * dout, torch.zeros_like(dout))
-        dy_complex, u = _rows(dy_complex, C.t()), _rows(u, B)
-        dscan = _proj(C, dy_complex, conj_transpose=True, padded=True)
+        dy_complex, kernel = _rows(dy_complex, C.t())
+        u, _ = _rows(u, B)
+        dscan = _proj(C, dy_complex, conj_transpose=True, padded=True, kernel=kernel)
         dC = _wgrad(dy_complex, scan_out)
         if dscan.stride(-1) != 1:
             dscan = dscan.contiguous()
+        kernel = projection.fits(B.t(), Bu)
         res = simplified_scan_cuda.bwd(Bu, delta, A_k, ident, ident, deltaA, dscan, xs, ctx.discretization,
                                       need_dB_dC=False, out_=scan_out if scan_out.stride(-1) == 1 else None,
-                                      padded=projection.fits(B.t(), Bu))
+                                      padded=kernel)
         dBu, ddelta, dA = res[0], res[1], res[2]
         ddeltaA = res[5] if ctx.has_deltaA else None
-        du_scan = _proj(B, dBu, conj_transpose=True)
+        du_scan = _proj(B, dBu, conj_transpose=True, kernel=kernel)
         dB = _wgrad(dBu, u) if u.is_complex() else torch.einsum("bpl,bhl->ph", dBu, u.conj())
         if u.is_complex():
             du = du_scan + torch.complex(du_skip, torch.zeros_like(du_skip))

@@ -120,3 +120,67 @@ def test_infinities_and_nans(M, K, N):
     b[:, 1] = 1 + 0.5j
     a[0, 3, 5], a[1, M - 1, N - 1], b[1, K - 1, 0] = complex(inf, 0), complex(1, nan), complex(0, -inf)
     _same_specials(projection.gradient(a, b), _plain("bml,bnl->mn", a, b.conj()))
+
+
+def _errors(got, want):
+    """(2-norm of the error over that of the result, the error's share along the result)"""
+    e = got.to(torch.complex128) - want
+    return float(e.norm() / want.norm()), float((want.conj() * e).sum().real / want.norm() ** 2)
+
+
+@pytest.mark.parametrize("real", [True, False])
+@pytest.mark.parametrize("K", [64, 80, 95, 96, 130, 384, 1000])
+def test_error_against_a_float32_product(K, real):
+    """The error is no larger than a float32 einsum's, and not to one side (an error to one side adds up over the scan
+    behind it; truncation in the accumulator alone would make 1.3e-7)."""
+    from lrnnx_b200.ops import projection
+    g = torch.Generator().manual_seed(K)
+    W, x = _cn(g, 100, K), _cn(g, 2, K, 2001)
+    if real:
+        x = torch.complex(x.real, torch.zeros_like(x.real))
+    want = torch.einsum("mk,bkn->bmn", W.to(torch.complex128), x.to(torch.complex128))
+    err, side = _errors(projection.product(W, x), want)
+    err32, _ = _errors(torch.einsum("mk,bkn->bmn", W, x), want)
+    assert err <= 1.02 * err32 and abs(side) <= 3e-8, (err, err32, side)
+
+
+@pytest.mark.parametrize("real", [True, False])
+@pytest.mark.parametrize("batch,L", [(1, 1024), (2, 1999)])
+def test_error_of_the_gradient_against_a_float32_product(batch, L, real):
+    from lrnnx_b200.ops import projection
+    g = torch.Generator().manual_seed(L)
+    a, b = _cn(g, batch, 100, L), _cn(g, batch, 50, L)
+    if real:
+        b = torch.complex(b.real, torch.zeros_like(b.real))
+    want = torch.einsum("bml,bnl->mn", a.to(torch.complex128), b.to(torch.complex128).conj())
+    err, side = _errors(projection.gradient(a, b), want)
+    err32, _ = _errors(torch.einsum("bml,bnl->mn", a, b.conj()), want)
+    assert err <= 1.02 * err32 and abs(side) <= 3e-8, (err, err32, side)
+
+
+@pytest.mark.parametrize("P,H,L,disc", [(192, 112, 81, "zoh"), (176, 328, 64, "dirac"), (56, 400, 515, "bilinear")])
+def test_simplified_scan_is_as_exact_as_with_einsums(P, H, L, disc, monkeypatch):
+    """The whole op against float64: an error of the products to one side would add up over the scan, and to the scan's
+    own (5 to 10 % more than with float32 einsums in place of the kernels)."""
+    from lrnnx_b200.ops import projection, simplified_scan_fn
+    from oracle import scan_oracle as O
+    g = torch.Generator().manual_seed(P)
+    r = lambda *s: torch.rand(*s, generator=g)  # noqa: E731
+    A = torch.log(torch.polar(0.9 + 0.099 * r(P), torch.pi / 10 * r(P)))
+    u = torch.complex(torch.randn(2, H, L, generator=g), torch.zeros(2, H, L))
+    t = [u, torch.ones(2, P, L) if disc == "dirac" else 0.5 + r(2, P, L), A, _cn(g, P, H).cpu() / H ** 0.5, _cn(g, H, P).cpu() / P ** 0.5]
+    gout = _cn(g, 2, H, L).cpu()
+
+    def run(fn, cast, **kw):
+        leaves = [cast(v).requires_grad_(True) for v in t]
+        y = fn(*leaves, discretization=disc, **kw)
+        return [y.detach().cpu()] + [v.cpu() for v in torch.autograd.grad(y, leaves, cast(gout))]
+
+    wide = lambda v: v.to(torch.complex128 if v.is_complex() else torch.float64)  # noqa: E731
+    want = run(O.simplified_scan_oracle, wide, compute_dtype=torch.float64)
+    err = lambda: [float((wide(a) - b).norm() / b.norm()) for a, b in zip(run(simplified_scan_fn, lambda v: v.cuda()), want)]  # noqa: E731
+    here = err()
+    monkeypatch.setattr(projection, "fits", lambda W, x: False)
+    monkeypatch.setattr(projection, "grad_fits", lambda g, u: False)
+    ratios = [a / b for a, b in zip(here, err())]
+    assert sum(ratios) / len(ratios) <= 1.02, ratios

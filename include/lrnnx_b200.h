@@ -79,11 +79,14 @@ typedef struct b200_selscan_fwd_args {
                                scanned from a zero state by its own thread blocks (more parallelism for
                                long rows); out, out_z and x of segments >= 1 are then zero-start results
                                that the caller must stitch with b200_selscan_fixup (n_segments = S).
+                               With seg_work: segments of seg_len steps, scanned in two passes; the results
+                               are those of the plain scan.
                                Honoured only on the shape class served by the state-parallel kernels,
                                rejected with B200_ERR_UNSUPPORTED elsewhere. */
   int32_t stage_len;        /* spacing in steps of the states in stage_h: the value returned by
                                b200_selscan_stage_states() for this problem (0 when stage_h is NULL) */
-  int32_t reserved0;
+  int32_t seg_len;          /* with seg_work: steps per segment, a multiple of 32, with l_segments * seg_len
+                               >= seqlen > (l_segments - 1) * seg_len */
   const void *u, *delta, *A, *B, *C;
   const void *D, *z, *delta_bias, *deltaA;      /* nullable */
   void *out;                                    /* (batch, dim, seqlen) */
@@ -104,6 +107,8 @@ typedef struct b200_selscan_fwd_args {
   int64_t A_ds, A_ns;
   int64_t B_bs, B_gs, B_ns;   /* variable: batch/group/state strides; constant: B_gs = dim stride */
   int64_t C_bs, C_gs, C_ns;
+  void *seg_work;             /* nullable: device workspace of l_segments * batch * dim * 17 floats, 16-byte aligned,
+                                 free again when the call's work on `stream` is done */
 } b200_selscan_fwd_args;
 
 int b200_selscan_fwd(const b200_selscan_fwd_args *args, void *stream);

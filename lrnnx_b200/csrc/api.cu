@@ -42,7 +42,7 @@ using namespace b200;
 extern "C" {
 
 const char *b200_last_error(void) { return g_err; }
-int b200_abi_version(void) { return 6; }
+int b200_abi_version(void) { return 7; }
 
 // size of an argument block as this library was compiled; lets a binding
 // verify its own struct layout before the first call
@@ -72,6 +72,12 @@ int b200_selscan_fwd(const b200_selscan_fwd_args *args, void *stream) {
   B200_REQUIRE(args->out && args->x, B200_ERR_NULL, "selscan_fwd: out and x must be non-null");
   B200_REQUIRE(!args->z || args->out_z, B200_ERR_NULL, "selscan_fwd: out_z is required when z is given");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (args->l_segments > 1 && args->seg_work) {
+    const int64_t S = args->l_segments, len = args->seg_len;
+    B200_REQUIRE(len > 0 && len % 32 == 0 && S * len >= args->seqlen && (S - 1) * len < args->seqlen, B200_ERR_SHAPE,
+                 "selscan_fwd: %d segments of %d steps do not make up %d", args->l_segments, args->seg_len, args->seqlen);
+    B200_REQUIRE((reinterpret_cast<uintptr_t>(args->seg_work) & 15) == 0, B200_ERR_ALIGN, "selscan_fwd: seg_work must be 16-byte aligned");
+  }
   if (selscan_seq_supported(*args)) {
     b200_selscan_fwd_args a = *args;
     if (a.stage_len != kStage) a.stage_h = nullptr;

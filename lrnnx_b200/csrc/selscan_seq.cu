@@ -18,6 +18,12 @@
 // 302 us; the SFU's floor: 110 us with softplus and gate).  1536 warps are 2.6 per scheduler: the rest is latency
 // (IPC 1.8 of 4, SFU 54 %, shared-memory pipe 57 %).  64 x 4096 x 512: 1.00 ms (1.52 ms).  Any length: a 4 x 776 x 1531
 // float32 call takes 90 us where the one-warp-per-row kernel that used to serve odd lengths took 1.1 ms.
+// Few rows: a step takes a thread block 60 ns however idle the GPU is, so a call whose blocks do not fill it is scanned in
+// segments, in two passes: states alone from zero for all segments but the last, then each segment from the state that
+// the ones before it lead to (the fold is a short loop at a block's start).  Nothing is corrected afterwards, and 16-bit
+// outputs are rounded once.  1 x 64 x 8192: 547 -> 25 us; 1 x 1536 x 512 bf16: 37 -> 18 us (a kernel that scans across lanes: 20).
+// The two passes cost 1.5 times one, so calls that fill the GPU are not cut like this.
+// Groups of at most 16 channels run in thread blocks of two warps: half of four would only help with the B | C tile.
 // Results match csrc/selective_scan/selective_scan.cuh:73-382 of lrnnx for this shape class.
 #include "selscan_seq.cuh"
 
@@ -25,16 +31,23 @@ namespace b200 {
 namespace {
 using namespace seq;
 
-constexpr int FW = 4;             // warps per thread block
 constexpr int TB = 4;             // steps per block of the recurrence
 
-// ALN: every row starts on a 16-byte boundary.  Z: gated.
-template <typename T, bool ALN, bool Z>
-__global__ void __launch_bounds__(FW * 32, 3) selscan_seq_fwd_kernel(const b200_selscan_fwd_args p) {
+// Segments of the sequence that are scanned side by side in two passes: the first leaves the state that a segment reaches
+// from zero and the sum of its step sizes, the second starts every segment from the state that the ones before it lead to.
+struct SeqSeg {
+  float4 *h;            // (segments, batch * dim, 4); null: a segment is a scan of its own, from a zero state
+  float *d;             // (segments, batch * dim)
+  int len;              // steps per segment
+};
+
+// ALN: every row starts on a 16-byte boundary.  Z: gated.  FW: warps per thread block.  SUM: the first pass of two.
+template <typename T, bool ALN, bool Z, int FW, bool SUM>
+__global__ void __launch_bounds__(FW * 32, 12 / FW) selscan_seq_fwd_kernel(const b200_selscan_fwd_args p, const SeqSeg seg) {
   constexpr int RAW = QCH * QT * (int)sizeof(T);                 // 8 rows of a stage
   __shared__ __align__(16) float bc_all[2][QT * QROW];           // B | C of a stage, float32, [t][n]
   __shared__ __align__(16) float dd_all[FW][QT * DROW];          // {delta, delta u} per (t, channel)
-  __shared__ __align__(16) float ys_all[FW][QT * QROW];          // partial outputs [t][channel][lane share]
+  __shared__ __align__(16) float ys_all[SUM ? 1 : FW][QT * QROW];       // partial outputs [t][channel][lane share]
   extern __shared__ __align__(16) unsigned char raw_all[];       // ALN: [warp][2 stages][u, delta, (z)] rows as they are
   constexpr int NRAW = Z ? 3 : 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -48,15 +61,9 @@ __global__ void __launch_bounds__(FW * 32, 3) selscan_seq_fwd_kernel(const b200_
   const int nch = min(cpg - cin, QCH);                           // <= 0: the warp only helps with the B | C tile
   const int d0 = g * cpg + cin;
   const int n_chunks = (p.seqlen + kChunk - 1) / kChunk;
-  // blockIdx.y = segment of the sequence, scanned from a zero state (whole checkpoint chunks)
-  int seg_len = p.seqlen;
-  if (gridDim.y > 1) {
-    const int per = (p.seqlen + (int)gridDim.y - 1) / (int)gridDim.y;
-    seg_len = ((per + kChunk - 1) / kChunk) * kChunk;
-  }
-  const int t_begin = (int)blockIdx.y * seg_len;
+  const int t_begin = (int)blockIdx.y * seg.len;                 // blockIdx.y = segment of the sequence
   if (t_begin >= p.seqlen) return;
-  const int L = min(p.seqlen, t_begin + seg_len);
+  const int L = min(p.seqlen, t_begin + seg.len);
   const int nst = (L - t_begin + QT - 1) / QT;
   const int dl = nch > 0 ? d0 : g * cpg;                         // a valid row for idle warps' pointers
 
@@ -73,18 +80,19 @@ __global__ void __launch_bounds__(FW * 32, 3) selscan_seq_fwd_kernel(const b200_
     Dp = reinterpret_cast<const T *>(p.delta) + (int64_t)b * p.delta_bs + (int64_t)dl * p.delta_ds + t_begin + lane;
     if (Z) Zp = reinterpret_cast<const T *>(p.z) + (int64_t)b * p.z_bs + (int64_t)dl * p.z_ds + t_begin + lane;
   }
-  // B | C: a thread takes 8 steps of one of the 32 rows
+  // B | C: a thread takes the same QT / FW steps of one of the 32 rows in every stage
+  constexpr int BCS = QT / FW;
   const T *BCp = lane < QN
       ? reinterpret_cast<const T *>(p.B) + (int64_t)b * p.B_bs + (int64_t)g * p.B_gs + (int64_t)lane * p.B_ns
       : reinterpret_cast<const T *>(p.C) + (int64_t)b * p.C_bs + (int64_t)g * p.C_gs + (int64_t)(lane - QN) * p.C_ns;
-  BCp += t_begin + 8 * warp;
-  constexpr int BCC = 8 / EPC<T>;
+  BCp += t_begin + BCS * warp;
+  constexpr int BCC = BCS / EPC<T>;
   uint4 rbc[BCC];
   auto load_stage = [&](int s) {
     const int left = L - (t_begin + s * QT);
 #pragma unroll
     for (int k = 0; k < BCC; ++k) {
-      rbc[k] = ld_chunk<T>(BCp + k * EPC<T>, left - 8 * warp - k * EPC<T>, ALN);
+      rbc[k] = ld_chunk<T>(BCp + k * EPC<T>, SUM && lane >= QN ? 0 : left - BCS * warp - k * EPC<T>, ALN);
     }
     BCp += QT;
     if constexpr (ALN) {
@@ -111,7 +119,7 @@ __global__ void __launch_bounds__(FW * 32, 3) selscan_seq_fwd_kernel(const b200_
   };
   load_stage(0);
 
-  float *dd = dd_all[warp], *ys = ys_all[warp];
+  float *dd = dd_all[warp], *ys = ys_all[SUM ? 0 : warp];
   float2 A2[2];
   {
     const float *A = reinterpret_cast<const float *>(p.A) + (int64_t)(dl + min(c, max(nch - 1, 0))) * p.A_ds;
@@ -128,7 +136,20 @@ __global__ void __launch_bounds__(FW * 32, 3) selscan_seq_fwd_kernel(const b200_
   }
   float2 h0 = make_float2(0.f, 0.f), h1 = h0;
   const bool mine = c < nch;
-  const int64_t row = (int64_t)b * p.dim + d0 + c;
+  const int64_t row = (int64_t)b * p.dim + d0 + c, n_rows = (int64_t)p.batch * p.dim;
+  float before = 0.f;                                            // sum of delta before the segment
+  if (!SUM && seg.h && mine) {
+    const float4 *hj = seg.h + row * 4 + q;
+    const float *dj = seg.d + row;
+#pragma unroll 4
+    for (int j = 0; j < (int)blockIdx.y; ++j, hj += n_rows * 4, dj += n_rows) {
+      const float4 hv = *hj;
+      const float d = *dj;
+      h0 = __ffma2_rn(ex2f2(__fmul2_rn(make_float2(d, d), A2[0])), h0, make_float2(hv.x, hv.y));
+      h1 = __ffma2_rn(ex2f2(__fmul2_rn(make_float2(d, d), A2[1])), h1, make_float2(hv.z, hv.w));
+      before += d;
+    }
+  }
 
   for (int s = 0; s < nst; ++s) {
     const int t0 = t_begin + s * QT;
@@ -140,7 +161,7 @@ __global__ void __launch_bounds__(FW * 32, 3) selscan_seq_fwd_kernel(const b200_
       float v[EPC<T>];
       unpack(rbc[k], v, T());
 #pragma unroll
-      for (int j = 0; j < EPC<T>; ++j) bc[(8 * warp + k * EPC<T> + j) * QROW + lane] = v[j];
+      for (int j = 0; j < EPC<T>; ++j) bc[(BCS * warp + k * EPC<T> + j) * QROW + lane] = v[j];
     }
     T uc[ALN ? 1 : QCH], zc[ALN ? 1 : QCH];
     float dv[QCH];
@@ -185,7 +206,7 @@ __global__ void __launch_bounds__(FW * 32, 3) selscan_seq_fwd_kernel(const b200_
           const int t = blk * TB + i;
           vd[i] = *reinterpret_cast<const float2 *>(dd + t * DROW + 2 * c);
           vb[i] = *reinterpret_cast<const float4 *>(bc + t * QROW + QS * q);
-          vc[i] = *reinterpret_cast<const float4 *>(bc + t * QROW + QN + QS * q);
+          if (!SUM) vc[i] = *reinterpret_cast<const float4 *>(bc + t * QROW + QN + QS * q);
         }
         float2 a0[TB], a1[TB];
 #pragma unroll
@@ -199,32 +220,37 @@ __global__ void __launch_bounds__(FW * 32, 3) selscan_seq_fwd_kernel(const b200_
           const float2 u2 = make_float2(vd[i].y, vd[i].y);
           h0 = __ffma2_rn(a0[i], h0, __fmul2_rn(u2, make_float2(vb[i].x, vb[i].y)));
           h1 = __ffma2_rn(a1[i], h1, __fmul2_rn(u2, make_float2(vb[i].z, vb[i].w)));
+          if (SUM) continue;
           const float2 y2 = __ffma2_rn(h1, make_float2(vc[i].z, vc[i].w), __fmul2_rn(h0, make_float2(vc[i].x, vc[i].y)));
           ys[(blk * TB + i) * QROW + 4 * c + q] = y2.x + y2.y;
         }
       }
-      if (p.stage_h && mine && (((t0 + QT) % p.stage_len) == 0 || s == nst - 1)) {
+      if (!SUM && p.stage_h && mine && (((t0 + QT) % p.stage_len) == 0 || t0 + QT >= p.seqlen)) {
         const int64_t n_stages = (p.seqlen + p.stage_len - 1) / p.stage_len;
         *reinterpret_cast<float4 *>(reinterpret_cast<float *>(p.stage_h) + (row * n_stages + t0 / p.stage_len) * QN + QS * q) =
             make_float4(h0.x, h0.y, h1.x, h1.y);
       }
     }
-    if (((t0 + QT) % kChunk) == 0 || s == nst - 1) {      // checkpoint
+    if (SUM ? s == nst - 1 : ((t0 + QT) % kChunk) == 0 || t0 + QT >= p.seqlen) {      // checkpoint, or the segment's summary
       float sum = 0.f;
 #pragma unroll
       for (int i = 0; i < QCH; ++i) {
         const float v = warp_sum(cs[i]);
         if (i == c) sum = v;
       }
-      if (mine) {
+      if (SUM && mine) {
+        seg.h[((int64_t)blockIdx.y * n_rows + row) * 4 + q] = make_float4(h0.x, h0.y, h1.x, h1.y);
+        if (q == 0) seg.d[(int64_t)blockIdx.y * n_rows + row] = sum;
+      } else if (mine) {
+        sum += before;
         float4 *xr = reinterpret_cast<float4 *>(reinterpret_cast<float *>(p.x) + (row * n_chunks + t0 / kChunk) * 2 * QN + 2 * QS * q);
         const float2 P0 = ex2f2(__fmul2_rn(make_float2(sum, sum), A2[0])), P1 = ex2f2(__fmul2_rn(make_float2(sum, sum), A2[1]));
         xr[0] = make_float4(P0.x, h0.x, P0.y, h0.y);
         xr[1] = make_float4(P1.x, h1.x, P1.y, h1.y);
       }
     }
-  
     __syncwarp();
+    if constexpr (SUM) continue;
     // ---- output: lane = timestep
     float yv[QCH];
 #pragma unroll
@@ -268,14 +294,16 @@ __global__ void __launch_bounds__(FW * 32, 3) selscan_seq_fwd_kernel(const b200_
           }
         }
     }
-  
     __syncwarp();
   }
 }
 
+// Warps per thread block: four share a B | C tile; a group of at most 16 channels has work for two.
+int warps_per_block(const b200_selscan_fwd_args &a) { return a.dim / a.n_groups > 2 * QCH ? 4 : 2; }
+
 int64_t fwd_blocks(const b200_selscan_fwd_args &a) {
-  const int cpg = a.dim / a.n_groups;
-  return (int64_t)a.batch * a.n_groups * ((cpg + FW * QCH - 1) / (FW * QCH));
+  const int cpg = a.dim / a.n_groups, per = warps_per_block(a) * QCH;
+  return (int64_t)a.batch * a.n_groups * ((cpg + per - 1) / per);
 }
 
 template <typename T> bool rows_aligned(const b200_selscan_fwd_args &a) {
@@ -284,24 +312,35 @@ template <typename T> bool rows_aligned(const b200_selscan_fwd_args &a) {
          (!a.z || (row16<T>(a.z, a.z_bs, a.z_ds) && row16<T>(a.out_z, a.out_z_bs, a.out_z_ds)));
 }
 
-// `operands`: how many of u, delta, z pass through shared memory as they are
-template <typename T, typename K>
-int launch_seq(K k, dim3 grid, int operands, const b200_selscan_fwd_args &a, cudaStream_t st) {
-  const int smem = FW * 2 * operands * QCH * QT * (int)sizeof(T);
+template <typename T, bool ALN, bool Z, int FW, bool SUM>
+int launch(const b200_selscan_fwd_args &a, const SeqSeg &seg, int segments, cudaStream_t st) {
+  auto k = selscan_seq_fwd_kernel<T, ALN, Z, FW, SUM>;
+  const int smem = ALN ? FW * 2 * (Z ? 3 : 2) * QCH * QT * (int)sizeof(T) : 0;      // u, delta, (z) as they are
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) { set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return (int)e; }
-  k<<<grid, FW * 32, smem, st>>>(a);
+  k<<<dim3((unsigned)fwd_blocks(a), (unsigned)segments), FW * 32, smem, st>>>(a, seg);
   return launch_status();
+}
+template <typename T, int FW> int launch_warps(const b200_selscan_fwd_args &a, const SeqSeg &seg, int segments, cudaStream_t st) {
+  const bool al = rows_aligned<T>(a);
+  if (seg.h)
+    if (int e = al ? launch<T, true, false, FW, true>(a, seg, segments - 1, st) : launch<T, false, false, FW, true>(a, seg, segments - 1, st)) return e;
+  if (a.z) return al ? launch<T, true, true, FW, false>(a, seg, segments, st) : launch<T, false, true, FW, false>(a, seg, segments, st);
+  return al ? launch<T, true, false, FW, false>(a, seg, segments, st) : launch<T, false, false, FW, false>(a, seg, segments, st);
 }
 
 template <typename T> int launch_fwd(const b200_selscan_fwd_args &a, cudaStream_t st) {
-  const dim3 grid((unsigned)fwd_blocks(a), (unsigned)(a.l_segments > 1 ? a.l_segments : 1));
   b200_selscan_fwd_args p = a;
-  if (a.l_segments > 1) p.stage_h = nullptr;      // segments start from zero: their states are not the sequence's
-  const bool al = rows_aligned<T>(a);
-  auto k = a.z ? (al ? selscan_seq_fwd_kernel<T, true, true> : selscan_seq_fwd_kernel<T, false, true>)
-               : (al ? selscan_seq_fwd_kernel<T, true, false> : selscan_seq_fwd_kernel<T, false, false>);
-  return launch_seq<T>(k, grid, al ? (a.z ? 3 : 2) : 0, p, st);
+  const int n = a.l_segments > 1 ? a.l_segments : 1;
+  SeqSeg seg{nullptr, nullptr, a.seqlen};
+  if (n > 1 && a.seg_work) {
+    const int64_t rows = (int64_t)a.batch * a.dim;
+    seg = {reinterpret_cast<float4 *>(a.seg_work), reinterpret_cast<float *>(a.seg_work) + (int64_t)n * rows * QN, a.seg_len};
+  } else if (n > 1) {
+    seg.len = ((a.seqlen + n - 1) / n + kChunk - 1) / kChunk * kChunk;      // whole checkpoint chunks
+    p.stage_h = nullptr;                          // segments start from zero: their states are not the sequence's
+  }
+  return warps_per_block(a) == 4 ? launch_warps<T, 4>(p, seg, n, st) : launch_warps<T, 2>(p, seg, n, st);
 }
 }  // namespace
 

@@ -144,29 +144,75 @@ def _segments_for(u, batch, dim, seqlen, dstate, n_groups, is_complex, var_B, va
         return 1
     if seqlen < 4 * CHUNK:
         return 1
-    idx = u.device.index if u.device.index is not None else torch.cuda.current_device()
-    if idx not in _SM_COUNT:
-        _SM_COUNT[idx] = torch.cuda.get_device_properties(idx).multi_processor_count
-    sms = _SM_COUNT[idx]
+    sms = _sm_count(u)
     if u.dtype != torch.float32:
         # 16-bit outputs behind a cut are rounded twice, by the segment and by the fix-up: the places of the cuts show
         # in the results, and calls without cuts are the more exact.  So only what has always been cut is (whole
         # tiles of 16 channels and 8 steps, in whole 16-byte pieces of rows), and where it has always been.
         return _segments_16bit(batch * dim // 16, seqlen, 8 * sms) if _whole_tiles(dim // n_groups, seqlen, rows) else 1
-    n_rows = batch * dim
-    ctas = batch * n_groups * -(-(dim // n_groups) // 32)       # thread blocks of 32 channels; 3 fit on an SM
-    if ctas >= 12 * sms:
+    blocks = _blocks(batch, dim, n_groups)
+    if blocks >= 12 * sms:
         return 1
-    # measured: a step of a thread block takes 60, 80 and 105 ns with one, two and three of them on an SM;
-    # the fix-up of a segment takes 6 ns per row
-    step_ns = (0, 60, 80, 105)
     best, best_ns = 1, None
     for S, seg_len in _cuts(seqlen):
-        full, rest = divmod(ctas * S, 3 * sms)
-        ns = (full * step_ns[3] + step_ns[-(-rest // sms)]) * seg_len + 6 * n_rows * (S - 1)
+        ns = _stitched_ns(blocks, S, seg_len, batch * dim, sms)
         if best_ns is None or ns < 0.95 * best_ns:
             best, best_ns = S, ns
     return best
+
+
+def _blocks(batch, dim, n_groups):
+    """Thread blocks of 32 channels, or what takes the place of one; 3 fit on an SM."""
+    channels = dim // n_groups
+    return batch * n_groups * -(-channels // 32) if channels > 16 else -(-batch * n_groups // 2)
+
+
+def _walk_ns(blocks, steps, sms):
+    # measured: a step of a thread block takes 60, 80 and 105 ns with one, two and three of them on an SM
+    step_ns = (0, 60, 80, 105)
+    full, rest = divmod(blocks, 3 * sms)
+    return (full * step_ns[3] + step_ns[-(-rest // sms)]) * steps
+
+
+def _stitched_ns(blocks, S, seg_len, rows, sms):
+    return _walk_ns(blocks * S, seg_len, sms) + 6 * rows * (S - 1)        # measured: the fix-up takes 6 ns per row and segment
+
+
+def _two_passes(u, batch, dim, seqlen, n_groups, S):
+    """(segments, steps per segment) where a forward call that would run in ``S`` segments (1: none) is faster in two
+    passes over shorter ones, else None.  The first pass walks the states of all segments but the last, the second
+    starts every segment from where the ones before it end: there is nothing to correct afterwards, so outputs are
+    rounded once, and segments may be as short as the idle part of the GPU asks for."""
+    return _two_passes_for(_blocks(batch, dim, n_groups), batch * dim, seqlen, S, _sm_count(u))
+
+
+@functools.lru_cache(maxsize=1024)
+def _two_passes_for(blocks, rows, seqlen, S, sms):
+    if blocks >= 3 * sms or seqlen < 256:
+        return None
+    seg_len = -(-(-(-seqlen // S)) // CHUNK) * CHUNK if S > 1 else seqlen
+    now = 1.12 * _stitched_ns(blocks, S, seg_len, rows, sms)
+    if S > 1:       # the last segment is shorter and fills gaps: between the longest walk and whole waves, 1.2 times the full GPU's rate
+        now = min(now, 1.12 * (max(_walk_ns(1, seg_len, sms), 1.2 * 105 * blocks * seqlen / (3 * sms)) + 6 * rows * (S - 1)))
+    best, best_ns = None, now
+    for want in (2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64):
+        seg_len = -(-(-(-seqlen // want)) // 32) * 32
+        n = -(-seqlen // seg_len)
+        if n < 2 or seg_len < 64:
+            break
+        # measured: the walks of both passes take 1.5 times one pass' step times (and a plain call 1.12 times them), a
+        # launch 4.5 us, the state of an earlier segment 0.1 us, a wave of thread blocks 3.6 us to start
+        ns = 1.5 * _walk_ns(blocks * n, seg_len, sms) + 4500 + 100 * n + 3600 * -(-blocks * n // (3 * sms))
+        if ns < best_ns:
+            best, best_ns = (n, seg_len), ns
+    return best if best_ns < 0.9 * now - 4000 else None       # the host's share of a second launch
+
+
+def _sm_count(u):
+    idx = u.device.index if u.device.index is not None else torch.cuda.current_device()
+    if idx not in _SM_COUNT:
+        _SM_COUNT[idx] = torch.cuda.get_device_properties(idx).multi_processor_count
+    return _SM_COUNT[idx]
 
 
 def _cuts(seqlen):
@@ -261,7 +307,14 @@ def fwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, delta_softplus, discret
             a.out_z_bs, a.out_z_ds, _ = out_z.stride()
         S = _segments_for(u, batch, dim, seqlen, dstate, n_groups, is_complex, var_B, var_C, deltaA_,
                           discretization_method_str, (u, delta, B, C, z_, out, out_z))
-        stage_len = _lib.lib().b200_selscan_stage_states(ctypes.byref(a)) if S <= 1 else 0
+        stage_len = _lib.lib().b200_selscan_stage_states(ctypes.byref(a))     # 256 where the state-parallel kernels take the call
+        two = _two_passes(u, batch, dim, seqlen, n_groups, S) if stage_len > 0 else None
+        if two:
+            S, a.seg_len = two
+            seg_work = torch.empty((S, batch * dim, dstate + 1), dtype=torch.float32, device=u.device)
+            a.seg_work = seg_work.data_ptr()
+        elif S > 1:
+            stage_len = 0
         x_numel = batch * dim * n_chunks * dstate * 2
         if stage_len > 0:
             flat = torch.empty(x_numel + _stage_numel(batch, dim, seqlen, dstate, stage_len), dtype=A.dtype,
@@ -280,9 +333,9 @@ def fwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, delta_softplus, discret
             except RuntimeError as e:
                 if "l_segments" not in str(e):
                     raise
-                S, a.l_segments = 1, 0       # operands that the state-parallel kernels do not take
+                S, a.l_segments = 1, 0       # checkpoints that the state-parallel kernels do not take
                 _lib.call("b200_selscan_fwd", a, _stream(u))
-            if S > 1:
+            if S > 1 and not two:
                 _stitch_segments(a, x, S, seqlen, u)
         else:
             _lib.call("b200_selscan_fwd", a, _stream(u))
@@ -346,7 +399,12 @@ def bwd(u, delta, A, B, C, D_, z_, delta_bias_, deltaA_, dout, x_, out_, dz_, de
         dD = torch.empty_like(D_) if D_ is not None else None
         ddelta_bias = torch.empty_like(delta_bias_) if delta_bias_ is not None else None
         # one launch for all the accumulators; each is a tensor of its own, which a caller may keep without the others
-        torch._foreach_zero_([t for t in (dA, dB, dC, dD, ddelta_bias) if t is not None])
+        sums = [dA, dB, dC]
+        if dD is not None:
+            sums.append(dD)
+        if ddelta_bias is not None:
+            sums.append(ddelta_bias)
+        torch._foreach_zero_(sums)
         ddeltaA = torch.empty_like(deltaA_) if deltaA_ is not None else None
 
         q = _lib.struct("b200_selscan_bwd_args")()

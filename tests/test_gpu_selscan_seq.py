@@ -237,7 +237,7 @@ def test_entering_state_and_adjoint_against_the_coverage_kernels(batch, dim, gro
 
 @pytest.mark.parametrize("dim,groups,L", [(20, 1, 5 * 2048 + 131), (42, 2, 4 * 2048 + 1), (33, 3, 4 * 2048)])
 @pytest.mark.parametrize("offset", [0, 1])
-def test_segments_at_odd_sizes(dim, groups, L, offset):
+def test_segments_at_odd_sizes(dim, groups, L, offset, monkeypatch):
     """A float32 call of few rows is cut into segments at any length, channel count and alignment: outputs, checkpoints
     and gradients against the same call in one piece."""
     from lrnnx_b200 import selective_scan_cuda as ext
@@ -250,12 +250,11 @@ def test_segments_at_odd_sizes(dim, groups, L, offset):
     rule = ext._segments_for
     seen = []
 
+    monkeypatch.setattr(ext, "_two_passes", lambda *a: None)
+
     def run(S):
-        ext._segments_for = lambda *a: seen.append(rule(*a)) or (seen[-1] if S is None else S)
-        try:
-            out, x, out_z = ext.fwd(*args, True, "mamba")
-        finally:
-            ext._segments_for = rule
+        monkeypatch.setattr(ext, "_segments_for", lambda *a: seen.append(rule(*a)) or (seen[-1] if S is None else S))
+        out, x, out_z = ext.fwd(*args, True, "mamba")
         return [out, out_z, x] + ext.bwd(*args, dout, x, out, None, True, False, "mamba")
 
     got, want = run(None), run(1)
@@ -281,3 +280,55 @@ def test_infinite_decay(L):
     for name, a, b in [("out", out_g, out_c), ("last state", last_g, last_c)] + [(k, gg[k], gc[k]) for k in ("u", "B", "C", "D", "z")]:
         assert bool(b.isfinite().all())
         assert_close(a.cpu(), b, rtol=GRAD_RTOL32, atol_scale=GRAD_ATOL32, name=name)
+
+
+@pytest.mark.parametrize("dim,groups,L", [(20, 1, 700), (33, 3, 2049), (40, 1, 4200), (16, 2, 257)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_two_passes(dim, groups, L, dtype, offset, monkeypatch):
+    """Segments that start from the states of the ones before them, of one stage, of several and of nearly the whole
+    sequence, in aligned and unaligned rows, gated and not: the results of the plain scan (float32 up to the rounding of
+    the products that carry a state over a segment), saved states and checkpoints included."""
+    from lrnnx_b200 import selective_scan_cuda as ext
+    t, g = _make_inputs(2, dim, 16, L, seed=L, dtype=dtype, groups=groups, with_z=L % 2 == 1)
+    c = {k: (v.cuda() if torch.is_tensor(v) else v) for k, v in t.items()}
+    for k in ("u", "delta", "B", "C"):
+        c[k] = torch.full((*c[k].shape[:-1], L + 3), float("nan"), device="cuda", dtype=dtype)[..., offset:offset + L].copy_(c[k])
+    args = (c["u"], c["delta"], c["A"], c["B"], c["C"], c["D"], c["z"], c["delta_bias"], None)
+    dout = torch.randn(2, dim, L, generator=g).to(dtype).cuda()
+    monkeypatch.setattr(ext, "_segments_for", lambda *a: 1)
+
+    def run(seg_len):
+        monkeypatch.setattr(ext, "_two_passes", lambda *a: seg_len and (-(-L // seg_len), seg_len))
+        out, x, *rest = ext.fwd(*args, True, "mamba")
+        ptr, stage_len = ext._stage_states_of(x, 2, dim, L, 16)
+        assert stage_len == 256
+        n = 2 * dim * -(-L // 256) * 16
+        states = torch.empty(0, dtype=torch.float32, device="cuda").set_(x.untyped_storage(), x.numel(), (n,)).clone()
+        grads = ext.bwd(*args, dout, x, out if rest else None, None, True, False, "mamba")
+        return [out] + rest, [x, states], grads
+
+    want = run(None)
+    f32 = dtype == torch.float32
+    for seg_len in (32, 64, 224, (L - 1) // 32 * 32):
+        got = run(seg_len)
+        # 16-bit outputs are rounded once: they differ where float32 results round apart, by a unit in the last place
+        for a, b in zip(got[0], want[0]):
+            if not f32:
+                assert float((a != b).float().mean()) < 0.02
+            assert_close(a.float().cpu(), b.float().cpu(), rtol=1e-5 if f32 else 2 ** -7, atol_scale=2e-6, name=f"{seg_len} output")
+        for a, b in zip(got[1], want[1]):
+            assert_close(a.cpu(), b.cpu(), rtol=1e-5, atol_scale=2e-6, name=f"{seg_len} states")
+        for i, (a, b) in enumerate(zip(got[2], want[2])):
+            assert_close(a.float().cpu(), b.float().cpu(), rtol=1e-4 if f32 else 3e-2, atol_scale=1e-5 if f32 else 1e-2, name=f"{seg_len} gradient {i}")
+
+
+def test_rule_of_the_two_passes():
+    """Few rows and a long sequence, at any length, alignment and type; not where the rows fill the GPU."""
+    from lrnnx_b200 import selective_scan_cuda as ext
+    u = torch.empty(1, device="cuda")
+    for batch, dim, L in ((1, 64, 32765), (1, 16, 131072), (2, 512, 16384), (1, 1536, 2048)):
+        S, seg_len = ext._two_passes(u, batch, dim, L, 1, 1)
+        assert seg_len % 32 == 0 and (S - 1) * seg_len < L <= S * seg_len
+    for batch, dim, L in ((8, 1536, 2048), (64, 4096, 512), (1, 64, 200)):
+        assert ext._two_passes(u, batch, dim, L, 1, 1) is None

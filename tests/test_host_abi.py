@@ -166,6 +166,20 @@ def test_projections_leave_operands_of_two_devices_to_torch():
     assert not projection.supported(W, x) and not projection.grad_supported(g, x)
 
 
+def test_segments_of_two_passes_make_up_the_sequence():
+    lib = _lib.lib()
+    buf = (ctypes.c_float * 64)()
+    a = _lib.struct("b200_selscan_fwd_args")()
+    a.u = a.delta = a.A = a.B = a.C = a.out = a.x = a.seg_work = -(-ctypes.addressof(buf) // 16) * 16
+    a.batch = a.dim = a.n_groups = a.var_B = a.var_C = 1
+    a.seqlen, a.dstate, a.method = 100, 16, _lib.enum("B200_DISC_MAMBA")
+    for S, seg_len in ((2, 32), (2, 50), (4, 96), (3, 0), (2, -64), (1 << 20, 1 << 30)):
+        a.l_segments, a.seg_len = S, seg_len
+        assert lib.b200_selscan_fwd(ctypes.byref(a), None) == _lib.enum("B200_ERR_SHAPE")
+    a.l_segments, a.seg_len, a.seg_work = 4, 32, a.seg_work + 4
+    assert lib.b200_selscan_fwd(ctypes.byref(a), None) == _lib.enum("B200_ERR_ALIGN")
+
+
 def test_install_registers_extension_modules():
     import sys
     import lrnnx_b200

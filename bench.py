@@ -24,9 +24,10 @@ x_k = Lambda x_{k-1} + (B u)_k  (A = log Lambda, delta = 1, "dirac").
              host cores on a bounded sample of the same workload.
 
   workloads  the default run adds one sub-record per further workload (lm_cfg2: configs[2] LM training
-             step; decode_cfg4: configs[4] generation; and the kernel-level ones below), each with
-             its own ms_per_step, value, roofline, kernels, e2e and cpu_baseline (fewer steps each,
-             so that the whole run stays within a few minutes): s6_cfg0, s6_layer and
+             step; decode_cfg4: configs[4] generation; and the kernel-level ones below) with its value,
+             unit, ms_per_step and e2e value; the whole record of each, with clocks, roofline, kernels
+             and cpu_baseline, is a line of its own on stderr, so that the result line stays short
+             (fewer steps each, so that the whole run stays within a few minutes): s6_cfg0, s6_layer and
              s6_layer_f32 (one Mamba layer's scan at the configs[2] shape), s6_long (configs[3];
              sequence-parallel with a correctness check of the stitched output when N > 1),
              ssu_step (configs[4] state-update kernels), cauchy, s5_scan_zoh (configs[1] with a
@@ -1386,6 +1387,18 @@ def measure(wl, steps, warmup, world, rank, local, dev, pg, sample_clocks=True):
     return rec
 
 
+def result_line(line, subs):
+    """The line for stdout: the top-level record, and of each further workload what a reader compares first.  Whole records
+    are some 17 KB, more than those who read the line keep of it."""
+    short = {k: v for k, v in line.items() if k != "kernels"}
+    if subs:
+        short["workloads"] = {
+            name: {"value": float("%.6g" % r["value"]), "unit": r["unit"], "ms_per_step": float("%.4g" % r["ms_per_step"]),
+                   "e2e": float("%.6g" % r["e2e"]["value"]), **({"sp_check": r["sp_check"]["ok"]} if r.get("sp_check") else {})}
+            for name, r in subs.items()}
+    return json.dumps(short)
+
+
 def run_ours(args, wl, with_subs):
     world = int(os.environ.get("WORLD_SIZE", "1"))
     rank = int(os.environ.get("RANK", "0"))
@@ -1405,10 +1418,11 @@ def run_ours(args, wl, with_subs):
         guard.start()
         torch.distributed.init_process_group("nccl", device_id=dev)
         pg = torch.distributed.group.WORLD
+    wl_name = wl.name
     line = measure(wl, args.steps, args.warmup, world, rank, local, dev, pg)
     failed = False
+    subs = {}
     if with_subs:
-        subs = {}
         names = SUB_WORKLOADS + (("s5_strong",) if world > 1 else ())
         del wl
         for name in names:
@@ -1425,8 +1439,6 @@ def run_ours(args, wl, with_subs):
                 if rec.get("sp_check") is not None and not rec["sp_check"]["ok"]:
                     failed = True
             del sub
-        if rank == 0:
-            line["workloads"] = subs
     elif rank == 0 and line.get("sp_check") is not None and not line["sp_check"]["ok"]:
         failed = True
     if world > 1:
@@ -1437,7 +1449,9 @@ def run_ours(args, wl, with_subs):
         torch.distributed.barrier()
         torch.cuda.synchronize()
     if rank == 0:
-        emit(json.dumps(line))
+        for name, rec in {wl_name: line, **subs}.items():
+            sys.stderr.write(json.dumps({"workload": name, **rec}) + "\n")
+        emit(result_line(line, subs))
     if failed:
         sys.stderr.write("bench.py: the sequence-parallel output differs from the unsplit forward (sp_check)\n")
     if world > 1:

@@ -46,9 +46,10 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a
 // Both terms of a conjugate pair share the real part dr of z - w and z - conj(w); with e1 = zi - wi, e2 = zi + wi
 //     v / (z - w) + conj(v) / (z - conj(w)) = v (dr, -e1) / (dr^2 + e1^2) + conj(v) (dr, -e2) / (dr^2 + e2^2)
 // are 18 fp32 operations beside two reciprocals (16 cycles of the SFU); as two complex reciprocals and products they
-// were 24.  The two reciprocals stay two (a common denominator would cancel near the poles), and v multiplies the
+// were 24.  The reciprocals' parts are added before they meet v: an output's running sum is then rounded twice per pole and
+// part, an error of 1.7e-7 (four chained multiply-adds: 2.4e-7, at the same number of operations).  The two reciprocals stay two (a common denominator would cancel near the poles), and v multiplies the
 // finished reciprocal (v dr could overflow where the quotient does not).  Two positions per packed instruction halve
-// the issue slots.  1024 rows, 32 poles, L = 4096: 117 -> 82 us (67 us are the fp32 pipe's floor, 58 the SFU's).
+// the issue slots.  1024 rows, 32 poles, L = 4096: 117 -> 79 us (67 us are the fp32 pipe's floor, 58 the SFU's).
 __global__ void __launch_bounds__(CT) cauchy_fwd_kernel(const cf *__restrict__ v, const cf *__restrict__ z,
                                                         const cf *__restrict__ w, cf *__restrict__ out, int n, int L) {
   __shared__ float4 vw[NMAX_SMEM];
@@ -162,8 +163,8 @@ __global__ void __launch_bounds__(BTT) s4_bwd_partial_kernel(const cf *__restric
     // Positions l and l + BTT packed.  With dr, e1, e2 as in the forward and g = dout
     //     s1 = g (dr, e1) / m1,  s2 = conj(g) (dr, -e2) / m2,   dv += s1 + s2
     //     dw += s1 (dr, e1) / m1 + s2 (dr, -e2) / m2
-    // 32 fp32 operations and two reciprocals.  1024 rows, 32 poles, L = 4096: 227 -> 177 us (119 us are the fp32
-    // pipe's floor).
+    // 34 fp32 operations and two reciprocals; the terms are formed before they are added.  1024 rows, 32 poles, L = 4096:
+    // 227 -> 182 us (127 us are the fp32 pipe's floor).
     float2 b1r[TN], b1i[TN], b2r[TN], b2i[TN];
 #pragma unroll
     for (int k = 0; k < TN; ++k) b1r[k] = b1i[k] = b2r[k] = b2i[k] = make_float2(0.f, 0.f);

@@ -1,15 +1,15 @@
 // Selective scan with one state per channel and constant B and C, float32: the RG-LRU and S7 layers
 // (lrnnx/ops/rglru_scan.py:28-144, lrnnx/ops/s7_scan.py:28-180 call the extension this way).
 //
-// With a single state nothing is reused: the kernel is bound by HBM (12 bytes a step forward, 20 backward),
-// so time is what threads share.  A thread block owns a row and takes 2048 steps (one checkpoint chunk) at a
+// With a single state nothing is reused (12 bytes a step forward, 20 backward), and what a step costs is instructions: the
+// coefficient, the scans and the way through shared memory (IPC 3.5 of 4 forward, 2.5 backward; DRAM 27 %).  A thread block owns a row and takes 2048 steps (one checkpoint chunk) at a
 // time, 256 per warp, 8 consecutive ones per lane; rows of up to 256, 512 and 1024 steps get 1, 2 and 4 warps.
 // Rows are read and written by coalesced 4-byte elements and turned to 8 steps per lane through a conflict-free
 // row in shared memory: any length and alignment.  Thread-serial scan of 8 steps, warp-shuffle scan of the
 // lanes, a short fold over the warps.  The backward rebuilds the states from the checkpoint before the chunk and
 // runs the adjoint in the same pass: g_t = dy_t B C + q_t, q_{t-1} = a_t g_t.
-// Measured, 4 x 1024 rows x 2048 steps: forward 29 us, backward 59 us (the one-warp-per-row coverage kernels: 151 and
-// 378 us; the bytes alone: 15 and 25 us at the copy rate).
+// Measured, 4 x 1024 rows x 2048 steps: forward 32 us, backward 61 us (the one-warp-per-row coverage kernels: 151 and
+// 378 us; the bytes alone: 15 and 25 us at the copy rate).  The exponential beside expm1 is 2 us of each.
 // The RG-LRU input gain sqrt(1 - a^2) is taken from expm1, which keeps it exact where a is close to 1; the transition
 // itself is the exponential where it is small (dA is divided by A, so a's error counts relative to a).
 #include "common.cuh"

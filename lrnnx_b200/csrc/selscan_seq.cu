@@ -16,7 +16,7 @@
 //   * the state at the end of every stage_len steps is an optional output (stage_h) for the backward.
 // Measured, batch 8 x 1536 channels x 2048 steps, bf16, gated: 220 us (a kernel that scans across the lanes of a warp:
 // 302 us; the SFU's floor: 110 us with softplus and gate).  1536 warps are 2.6 per scheduler: the rest is latency
-// (IPC 1.8 of 4, SFU 54 %, shared-memory pipe 57 %).  64 x 4096 x 512: 1.00 ms (1.52 ms).  Any length: a 4 x 776 x 1531
+// (IPC 1.8 of 4, SFU 56 %, shared-memory pipe 61 %).  64 x 4096 x 512: 1.00 ms (1.52 ms).  Any length: a 4 x 776 x 1531
 // float32 call takes 90 us where the one-warp-per-row kernel that used to serve odd lengths took 1.1 ms.
 // Few rows: a step takes a thread block 60 ns however idle the GPU is, so a call whose blocks do not fill it is scanned in
 // segments, in two passes: states alone from zero for all segments but the last, then each segment from the state that

@@ -13,8 +13,8 @@
 //      shuffles at every step).  delta, delta u and dy of 4 channels at a time are prepared once by
 //      all threads; the sums over the states (for du and ddelta) meet in shared memory.
 // Measured, batch 8 x 1536 channels x 2048 steps, bf16, gated: 280 + 415 us (a kernel that owns channels and scans
-// across lanes: 845 us).  The first launch is bound by its serial walks and the shared-memory pipe (75 %), the second by latency
-// (12 warps per SM, IPC 1.9 of 4, FMA pipe 43 %).  Blocks of 4 steps rather than 8: with 8 a lane needs 255 registers,
+// across lanes: 845 us).  The first launch is bound by the shared-memory pipe (93 %; SFU 76 %), the second by latency
+// (12 warps per SM, IPC 1.9 of 4, FMA pipe 44 %).  Blocks of 4 steps rather than 8: with 8 a lane needs 255 registers,
 // two warps per scheduler are left and the second launch takes 600 us, for 90 us less in the first.
 // Gradients of A, B, C, D and delta_bias leave by float32 atomics, one per (n, t) and run of
 // channels for B and C, one per (channel, n) and 128 steps for A.
